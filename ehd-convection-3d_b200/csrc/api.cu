@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "ehd.h"
+#include "column.h"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -269,6 +270,51 @@ int poisson(ehd_ctx *c) {
     return EHD_OK;
 }
 
+// Whether the context's next steps run on the column kernel: a 1 x 1 x NZ grid
+// in the steady state, unless the per-node kernel was asked for.
+bool on_column(const ehd_ctx *c) {
+    return column_usable(c->p.nx, c->p.ny, c->p.nz) && c->tune.lbm_kernel == 0 &&
+           c->have_state && !c->pops_local && !c->e_arrays;
+}
+
+// nsteps steady-state steps of a column, launches of up to kColumnSteps.  At
+// about a microsecond a step a launch lasts milliseconds: its few microseconds
+// of set-up (the state read and written once) do not count, and other work on
+// the device is not held up for longer.
+constexpr int kColumnSteps = 4096;
+int column_steps(ehd_ctx *c, int nsteps) {
+    while (nsteps > 0) {
+        const int m = std::min(nsteps, kColumnSteps);
+        ColumnArgs a{};
+        for (int i = 0; i < 2; ++i) {
+            a.f[i] = c->f[i];
+            a.h[i] = c->h[i];
+            a.wref[i] = c->wref[i];
+            a.mean[i] = c->mean[i];
+            a.ktab[i] = c->ktab[i];
+        }
+        a.phip = c->phip;
+        a.q = c->q;
+        a.rho = c->rho;
+        a.u = c->u;
+        a.v = c->v;
+        a.w = c->w;
+        a.phi00 = c->phi00;
+        a.ez00 = c->ez00;
+        a.dz = c->p.dz;
+        a.eps = c->p.eps;
+        a.voltage = c->p.voltage;
+        a.parity = c->cur;
+        cudaError_t e = launch_column_steps(c->prec, a, c->sc, m, c->stream);
+        if (e != cudaSuccess) return fail(EHD_ERR_CUDA, "column step launch: %s", cudaGetErrorString(e));
+        c->cur ^= m & 1;
+        c->step += m;
+        for (int i = 0; i < m; ++i) c->t += c->p.dt;
+        nsteps -= m;
+    }
+    return EHD_OK;
+}
+
 void drop_graphs(ehd_ctx *c) {
     for (auto &row : c->graph)
         for (auto &g : row)
@@ -374,6 +420,7 @@ cudaStream_t ctx_stream(const ehd_ctx *c) { return c->stream; }
 int ctx_device(const ehd_ctx *c) { return c->device; }
 int ctx_precision(const ehd_ctx *c) { return c->prec; }
 bool ctx_steady(const ehd_ctx *c) { return c->have_state && !c->pops_local && !c->e_arrays; }
+bool ctx_column(const ehd_ctx *c) { return on_column(c); }
 int ctx_parity(const ehd_ctx *c) { return c->cur; }
 int ctx_launch_step(ehd_ctx *c, bool macros) {
     const int cur0 = c->cur;
@@ -538,6 +585,10 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
             default: e = prepare_lbm_rows<__nv_bfloat16, float>(nx, ny, nz, &c->rows_grid); break;
         }
         if (e != cudaSuccess) return bail(fail(EHD_ERR_CUDA, "row kernel set-up: %s", cudaGetErrorString(e)));
+    }
+    if (column_usable(nx, ny, nz)) {
+        cudaError_t e = prepare_column(c->prec);
+        if (e != cudaSuccess) return bail(fail(EHD_ERR_CUDA, "column kernel set-up: %s", cudaGetErrorString(e)));
     }
     {
         // room for the plane sums of every launch shape ehd_set_tuning allows
@@ -844,6 +895,10 @@ int ehd_step(ehd_ctx *c, int nsteps) {
     for (int i = 0; i < nsteps; ++i) {
         const bool macros = (i == nsteps - 1);
         int r;
+        if (on_column(c)) {  // all remaining steps at once
+            if ((r = column_steps(c, nsteps - i)) != EHD_OK) return r;
+            break;
+        }
         if (c->pops_local || c->e_arrays || !c->use_graphs) {
             if ((r = lbm(c, macros)) != EHD_OK) return r;
             if ((r = poisson(c)) != EHD_OK) return r;

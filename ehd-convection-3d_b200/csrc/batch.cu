@@ -283,6 +283,24 @@ int order(ehd_batch *b, const std::vector<char> &act, bool to_batch) {
     return e == cudaSuccess ? EHD_OK : cuda_fail("batch stream order", e);
 }
 
+// steps k .. nsteps - 1 of the active instances, one graph launch each
+int graph_steps(ehd_batch *b, const std::vector<char> &act, int k, int nsteps) {
+    int r = order(b, act, true);
+    for (; r == EHD_OK && k < nsteps; ++k) {
+        cudaGraphExec_t ge = nullptr;
+        if ((r = step_graph(b, act, k == nsteps - 1, &ge)) != EHD_OK) break;
+        cudaError_t e = cudaGraphLaunch(ge, b->stream);
+        if (e != cudaSuccess) {
+            r = cuda_fail("batch graph launch", e);
+            break;
+        }
+        for (size_t i = 0; i < b->inst.size(); ++i)
+            if (act[i]) ctx_commit_step(b->inst[i]);
+    }
+    const int r2 = order(b, act, false);
+    return r != EHD_OK ? r : r2;
+}
+
 int batch_step(ehd_batch *b, const std::vector<char> &act, int nsteps) {
     int k = 0;
     bool any = false, general = false;
@@ -303,20 +321,22 @@ int batch_step(ehd_batch *b, const std::vector<char> &act, int nsteps) {
         k = 1;
     }
     if (k >= nsteps) return EHD_OK;
-    int r = order(b, act, true);
-    for (; r == EHD_OK && k < nsteps; ++k) {
-        cudaGraphExec_t ge = nullptr;
-        if ((r = step_graph(b, act, k == nsteps - 1, &ge)) != EHD_OK) break;
-        cudaError_t e = cudaGraphLaunch(ge, b->stream);
-        if (e != cudaSuccess) {
-            r = cuda_fail("batch graph launch", e);
-            break;
+    // columns take all their steps on their own streams, one launch each (a
+    // block per column, side by side); the graph steps the others
+    std::vector<char> rest = act;
+    any = false;
+    for (size_t i = 0; i < b->inst.size(); ++i) {
+        if (!act[i]) continue;
+        if (ctx_column(b->inst[i])) {
+            rest[i] = 0;
+            int r = ehd_step(b->inst[i], nsteps - k);
+            if (r != EHD_OK) return r;
+        } else {
+            any = true;
         }
-        for (size_t i = 0; i < b->inst.size(); ++i)
-            if (act[i]) ctx_commit_step(b->inst[i]);
     }
-    const int r2 = order(b, act, false);
-    return r != EHD_OK ? r : r2;
+    if (!any) return EHD_OK;
+    return graph_steps(b, rest, k, nsteps);
 }
 
 }  // namespace

@@ -229,6 +229,9 @@ cudaStream_t ctx_stream(const ::ehd_ctx *c);
 int ctx_device(const ::ehd_ctx *c);
 int ctx_precision(const ::ehd_ctx *c);
 bool ctx_steady(const ::ehd_ctx *c);
+// whether its next steps run on the column kernel (ehd_step then launches all
+// of them at once, so a batch leaves such an instance to its own stream)
+bool ctx_column(const ::ehd_ctx *c);
 int ctx_parity(const ::ehd_ctx *c);
 int ctx_launch_step(::ehd_ctx *c, bool macros);
 void ctx_commit_step(::ehd_ctx *c);
