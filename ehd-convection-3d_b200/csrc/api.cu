@@ -634,13 +634,21 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     if ((r = dalloc(c, &twx, (size_t)nx * c2))) return bail(r);
     if ((r = dalloc(c, &twy, (size_t)ny * c2))) return bail(r);
     const size_t nmodes = (size_t)pa.nxh * ny;
-    // z solve: sine transform, with compile-time FFT passes where 2 (nz - 1)
-    // is one of their sizes and run-time ones where the transforms of a few
-    // modes fit in shared memory; else the Thomas solve with its pivot table
-    // and sweep scratch
+    // BF16 storage keeps the run-time radix passes where there are no
+    // compile-time ones: such a run turns any change of FP32 round-off into a
+    // change as large as its own storage error (200 steps of a grid without
+    // compile-time passes moved v by 1.1e-2 of its norm on the folded
+    // transforms, each run being 8.5e-3 off the 64-bit one), and its results
+    // stay what they were.
+    const bool keep_rt = c->prec == EHD_PREC_BF16;
+    // z solve: the sine transform where 2 (nz - 1) is a compile-time FFT size;
+    // elsewhere the Thomas solves, with their pivot table and the FP64 sweep's
+    // scratch (ehd_tuning.z_solve)
     const int lz2 = 2 * (nz - 1);
-    bool zdst = poisson_fast_size(lz2);
-    if (!zdst) {
+    const bool thomas = !poisson_fast_size(lz2);
+    bool zdst = !thomas;
+    pa.ztb = 0;
+    if (thomas && keep_rt) {
         int tb = 16;
         while (tb > 1 && zdst_rt_smem(lz2, tb, c->rsize) > 160 * 1024) tb >>= 1;
         if (zdst_rt_smem(lz2, tb, c->rsize) <= 160 * 1024) {
@@ -649,9 +657,16 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
             pa.pz = make_plan(lz2);
         }
     }
-    // where 2 (nz - 1) is not a compile-time size, the Thomas solve stays
-    // available beside the run-time sine transform (ehd_tuning.z_solve)
-    const bool thomas = !poisson_fast_size(lz2);
+    // axes without compile-time passes: folded products, with the axis's table
+    // and, for y, a second spectrum
+    const bool dftx = !poisson_fast_size(nx) && dft_usable(nx, false, c->rsize) && !keep_rt;
+    const bool dfty = !poisson_fast_size(ny) && dft_usable(ny, true, c->rsize) && !keep_rt;
+    void *tabx = nullptr, *taby = nullptr;
+    if (dftx && (r = dalloc(c, &tabx, dft_table_elems(nx, false, c->rsize) * c2))) return bail(r);
+    if (dfty) {
+        if ((r = dalloc(c, &taby, dft_table_elems(ny, true, c->rsize) * c2))) return bail(r);
+        if ((r = dalloc(c, &pa.spec2, nspec * c2))) return bail(r);
+    }
     double *cpt = nullptr;
     void *twz = nullptr, *cps = nullptr;
     const bool split = poisson_split_grid(nx, ny, nz, c->rsize);
@@ -668,6 +683,8 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     pa.twx = twx;
     pa.twy = twy;
     pa.twz = twz;
+    pa.tabx = tabx;
+    pa.taby = taby;
     pa.lx = params->lx;
     pa.ly = params->ly;
     pa.cpt = cpt;
@@ -697,6 +714,16 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
             std::vector<float> tf(t.begin(), t.end());
             return cudaMemcpy(dst, tf.data(), sizeof(float) * 2 * N, cudaMemcpyHostToDevice);
         };
+        auto folded = [&](int N, bool y, void *dst) -> cudaError_t {
+            std::vector<double> t(2 * dft_table_elems(N, y, c->rsize));
+            dft_table(N, y, c->rsize, t.data());
+            if (c->rsize == 8)
+                return cudaMemcpy(dst, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice);
+            std::vector<float> tf(t.begin(), t.end());
+            return cudaMemcpy(dst, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice);
+        };
+        if (dftx) EHD_CK(folded(nx, false, tabx));
+        if (dfty) EHD_CK(folded(ny, true, taby));
         EHD_CK(table(nx, twx));
         EHD_CK(table(ny, twy));
         if (zdst) {

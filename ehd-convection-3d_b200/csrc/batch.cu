@@ -106,7 +106,7 @@ int build_group(ehd_batch *b, const std::vector<size_t> &members, bool macros,
         PoissonArgs pa{};
         int r = ctx_step_args(b->inst[members[m]], macros, &la[m], &sc[m], &rd[m], &pa);
         if (r != EHD_OK) return r;
-        pp[m] = PoissonPtrs{pa.spec, pa.rowsum, pa.planesum, pa.phi00, pa.ez00,
+        pp[m] = PoissonPtrs{pa.spec, pa.spec2, pa.rowsum, pa.planesum, pa.phi00, pa.ez00,
                             pa.q, pa.qmean, pa.phip, pa.dpw};
         if (m == 0) pa0 = pa;
     }
@@ -115,8 +115,10 @@ int build_group(ehd_batch *b, const std::vector<size_t> &members, bool macros,
     unsigned char *ld = nullptr;
     int r = upload(host.data(), host.size(), bufs, &ld);
     if (r == EHD_OK) r = upload(rd.data(), rd.size(), bufs, &g->red);
-    PoissonPtrs *pd = nullptr;
+    PoissonPtrs *pd = nullptr, *pd2 = nullptr;
     if (r == EHD_OK) r = upload(pp.data(), pp.size(), bufs, &pd);
+    for (PoissonPtrs &x : pp) x.spec = x.spec2;  // the z solve's buffer where y is folded
+    if (r == EHD_OK) r = upload(pp.data(), pp.size(), bufs, &pd2);
     if (r != EHD_OK) return r;
     const ehd_params *p = ctx_params(b->inst[members[0]]);
     g->nx = p->nx;
@@ -130,6 +132,7 @@ int build_group(ehd_batch *b, const std::vector<size_t> &members, bool macros,
     g->lbm = ld;
     g->pa = pa0;
     g->pa.grp = pd;
+    g->pa.grp2 = pd2;
     g->pa.ngrp = n;
     return EHD_OK;
 }
@@ -591,11 +594,12 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
             t.poisson_path = 1 - best.poisson_path;
             r = trial(t);
         }
-        if (r == EHD_OK && !poisson_fast_size(2 * (p.nz - 1))) {  // sine transform or Thomas
+        if (r == EHD_OK && !poisson_fast_size(2 * (p.nz - 1))) {  // which Thomas solve
             ehd_tuning t = best;
             t.z_solve = 1 - best.z_solve;
             r = trial(t);
         }
+        // run-time radix passes
         if (!poisson_fast_size(p.nx))
             for (int rows = 1; r == EHD_OK && rows <= 32; rows *= 2) {
                 ehd_tuning t = best;

@@ -128,6 +128,20 @@ inline cudaError_t allow_max_dynamic_smem(K kern) {
     return e;
 }
 
+// Opt in to more than 48 KB of dynamic shared memory (to the device's
+// maximum, see allow_max_dynamic_smem).  Skipped while the stream is being
+// captured into a graph: the attribute is set by the first, uncaptured launch
+// on the device.
+template <typename K>
+inline cudaError_t set_smem(K kern, size_t bytes, cudaStream_t s) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &st);
+    if (e != cudaSuccess) return e;
+    if (st != cudaStreamCaptureStatusNone) return cudaSuccess;
+    return allow_max_dynamic_smem(kern);
+}
+
 template <typename T> struct Store;
 template <> struct Store<double> {
     __device__ __forceinline__ static double ld(const double *p) { return __ldg(p); }

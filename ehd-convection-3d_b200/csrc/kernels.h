@@ -131,7 +131,7 @@ struct FftPlan {
 // instances with the same grid (blockIdx.z selects the instance); the tables
 // (twiddles, eigenvalues, pivots) are the same for the whole group.
 struct PoissonPtrs {
-    void *spec;
+    void *spec, *spec2;
     double *rowsum, *planesum, *phi00, *ez00;
     const void *q;
     const double *qmean;
@@ -145,17 +145,20 @@ struct PoissonPtrs {
 struct PoissonArgs {
     int nx, ny, nz, nxh, pitch;
     int split;           // 1: the split-y three-kernel path where it applies
-    int thomas;          // 1: the Thomas z solve where the sine transform is run-time
+    int thomas;          // 1: the FP64 Thomas sweep where L is not a compile-time size
     int rows_per_block;  // x-row FFT batch per block (run-time radix path)
     int cols_per_block;  // y-column FFT batch per block (run-time radix path)
     FftPlan px, py;
     const void *twx, *twy;   // exp(-2 pi i k/N) tables in the compute type
-    FftPlan pz;              // run-time plan of length L = 2 (nz - 1) (sine-transform
-                             // z solve when L is not a compile-time FFT size)
-    int ztb;                 // modes per block of that solve
-    const void *twz;         // sine-transform z solve, L = 2 (nz - 1), compute type:
-                             // exp(-2 pi i k/L) (L complex), then 4 sin^2(pi k/L)
-                             // (L/2 + 1 real); nullptr: Thomas solve
+    const void *tabx, *taby; // folded transforms (dft.cu): cosine and sine table of
+                             // the axis (dft_table) in the compute type, nullptr:
+                             // compile-time or run-time radix passes
+    FftPlan pz;              // run-time plan of length L = 2 (nz - 1) and modes per
+    int ztb = 0;             // block of the sine-transform z solve with run-time
+                             // passes; 0: compile-time ones
+    const void *twz;         // sine-transform z solve, compute type: exp(-2 pi i k/L)
+                             // (L complex), then 4 sin^2(pi k/L) (L/2 + 1 real);
+                             // nullptr: a Thomas solve with cpt
     double lx, ly;           // domain lengths (wavenumbers 2 pi k / l)
     const double *cpt;       // Thomas pivots [z-1][ky*nxh + kx], FP64
     const void *cps;         // split-y path: two-sided Thomas pivots [kx][j][r][k'] (ky = S k' + j,
@@ -163,6 +166,8 @@ struct PoissonArgs {
                              // in the compute type; nullptr: no split path
     double2 *dpw;            // FP64 scratch of the forward sweep, same layout
     void *spec;              // complex compute type
+    void *spec2;             // the same again where taby is set: the y transform goes
+                             // from spec to spec2 and back, the z solve runs in spec2
     double *rowsum;          // [z-1][y] FP64 sums of the source
     double *planesum;        // [z] FP64 sums of the source
     double *phi00, *ez00;    // [z] mean potential and its Ez
@@ -171,6 +176,7 @@ struct PoissonArgs {
     void *phip;              // output phi' (compute type)
     double eps, voltage, dz;
     const PoissonPtrs *grp = nullptr;  // device array: a launch over ngrp instances
+    const PoissonPtrs *grp2 = nullptr; // the same with spec = spec2 (where taby is set)
     int ngrp = 1;
 };
 
@@ -188,6 +194,24 @@ bool poisson_split_grid(int nx, int ny, int nz, size_t rsize);
 // shared memory of the run-time-radix sine-transform z solve with tb modes
 // per block (compute type of rsize bytes)
 size_t zdst_rt_smem(int L, int tb, size_t rsize);
+// ---- folded transforms and the z solve of any NZ (csrc/dft.cu) ----
+constexpr int kDftMax = 1024;
+// whether an axis of n points without compile-time passes is transformed by
+// folded products (else by run-time radix passes); y: the y passes
+bool dft_usable(int n, bool y, size_t rsize);
+// the axis's table in the order the kernels read it, pairs (cos, sin) of
+// 2 pi a b / n, zero padded: rows of dft_table_pitch pairs, dft_table_elems
+// pairs in all (y: the y passes' tiles; rsize: bytes of the compute type)
+int dft_table_pitch(int n, bool y, size_t rsize);
+size_t dft_table_elems(int n, bool y, size_t rsize);
+void dft_table(int n, bool y, size_t rsize, double *t);
+template <typename R> cudaError_t prepare_dft(int nx, int ny);
+template <typename R> cudaError_t launch_dft_rows_fwd(const PoissonArgs &a, cudaStream_t s);
+template <typename R> cudaError_t launch_dft_rows_inv(const PoissonArgs &a, cudaStream_t s);
+template <typename R> cudaError_t launch_dft_cols(const PoissonArgs &a, int sign, cudaStream_t s);
+// modes per block of the shared-memory z solve, 0: the columns do not fit
+int zmeet_modes(int nz, size_t rsize);
+template <typename R> cudaError_t launch_zmeet(const PoissonArgs &a, cudaStream_t s);
 
 // ---- diagnostics ---------------------------------------------------------
 

@@ -235,6 +235,8 @@ extern "C" int ehd_poisson_noalloc(const ehd_params *p, const double *q, double 
     a.eps = p->eps;
     a.voltage = p->voltage;
     a.dz = p->dz;
+    a.lx = p->lx;
+    a.ly = p->ly;
 
     const size_t nxy = (size_t)nx * ny;
     // every region the solve reads before writing is set here: the tables,

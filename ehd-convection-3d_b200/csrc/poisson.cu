@@ -1717,20 +1717,6 @@ poisson_rows_inv_split(const typename Cplx<R>::T *__restrict__ spl, R *__restric
 // launcher
 // ---------------------------------------------------------------------------
 
-// Opt in to more than 48 KB of dynamic shared memory (to the device's
-// maximum, see allow_max_dynamic_smem).  Skipped while the stream is being
-// captured into a graph: the attribute is set by the first, uncaptured launch
-// on the device.
-template <typename K>
-static cudaError_t set_smem(K kern, size_t bytes, cudaStream_t s) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(s, &st);
-    if (e != cudaSuccess) return e;
-    if (st != cudaStreamCaptureStatusNone) return cudaSuccess;
-    return allow_max_dynamic_smem(kern);
-}
-
 bool poisson_fast_size(int n) {
     return n == 48 || n == 64 || n == 80 || n == 96 || n == 128 || n == 256 || n == 512;
 }
@@ -1794,6 +1780,7 @@ static cudaError_t rows_fwd(const PoissonArgs &a, cudaStream_t s) {
         case 512: return rows_fwd_fast<R, 512>(a, s);
         default: break;
     }
+    if (a.tabx) return launch_dft_rows_fwd<R>(a, s);
     const int rows = a.rows_per_block;
     const size_t sm = (size_t)(2 * rows + 1) * a.nx * sizeof(R2);
     cudaError_t e = set_smem(poisson_rows_fwd<R>, sm, s);
@@ -1817,6 +1804,7 @@ static cudaError_t rows_inv(const PoissonArgs &a, cudaStream_t s) {
         case 512: return rows_inv_fast<R, 512>(a, s);
         default: break;
     }
+    if (a.tabx) return launch_dft_rows_inv<R>(a, s);
     const int rows = a.rows_per_block;
     const size_t sm = (size_t)(2 * rows + 1) * a.nx * sizeof(R2);
     cudaError_t e = set_smem(poisson_rows_inv<R>, sm, s);
@@ -1840,6 +1828,7 @@ static cudaError_t cols(const PoissonArgs &a, cudaStream_t s) {
         case 512: return cols_fast<R, 512, S>(a, s);
         default: break;
     }
+    if (a.taby) return launch_dft_cols<R>(a, S, s);
     const int cc = a.cols_per_block;
     const size_t sm = (size_t)(2 * cc + 1) * a.ny * sizeof(R2);
     cudaError_t e = set_smem(poisson_cols<R>, sm, s);
@@ -2082,6 +2071,7 @@ cudaError_t prepare_poisson(const PoissonArgs &a) {
     if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_rows_inv<R>);
     if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_cols<R>);
     if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_zdst_rt<R>);
+    if (e == cudaSuccess) e = prepare_dft<R>(a.nx, a.ny);
     if (e == cudaSuccess) e = prepare_fast<R>(a.nx);
     if (e == cudaSuccess) e = prepare_fast<R>(a.ny);
     if (e == cudaSuccess) e = prepare_fast<R>(2 * (a.nz - 1));
@@ -2103,9 +2093,52 @@ cudaError_t prepare_poisson(const PoissonArgs &a) {
 template cudaError_t prepare_poisson<float>(const PoissonArgs &);
 template cudaError_t prepare_poisson<double>(const PoissonArgs &);
 
+// The z solve of the general path, in the buffer that the forward y transform
+// left: the sine transform where L = 2 (NZ - 1) has compile-time passes, or
+// with run-time ones where the context keeps them (ztb > 0); otherwise the
+// two-sided Thomas solve with the columns in shared memory, or the FP64 sweep
+// through global memory where they do not fit or by choice.
+template <typename R>
+static cudaError_t zsolve(const PoissonArgs &a0, cudaStream_t s) {
+    using R2 = typename Cplx<R>::T;
+    PoissonArgs a = a0;
+    if (a.taby) {
+        a.spec = a0.spec2;
+        a.grp = a0.grp2;
+    }
+    if (a.twz && a.ztb == 0) {
+        switch (2 * (a.nz - 1)) {
+            case 48: return zdst<R, 48>(a, s);
+            case 64: return zdst<R, 64>(a, s);
+            case 80: return zdst<R, 80>(a, s);
+            case 96: return zdst<R, 96>(a, s);
+            case 128: return zdst<R, 128>(a, s);
+            case 256: return zdst<R, 256>(a, s);
+            default: return zdst<R, 512>(a, s);
+        }
+    }
+    const int modes = a.nxh * a.ny;
+    if (!a.thomas && a.twz) {  // run-time passes
+        const int L = 2 * (a.nz - 1);
+        const size_t sm = zdst_rt_smem(L, a.ztb, sizeof(R));
+        cudaError_t e = set_smem(poisson_zdst_rt<R>, sm, s);
+        if (e != cudaSuccess) return e;
+        const R2 *tw = (const R2 *)a.twz;
+        poisson_zdst_rt<R><<<dim3((modes + a.ztb - 1) / a.ztb, 1, a.ngrp), 256, sm, s>>>(
+            (R2 *)a.spec, tw, (const R *)(tw + L), a.pz, a.planesum, a.qmean, a.phi00, a.ez00,
+            a.nx, a.ny, a.nxh, a.pitch, a.ztb, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx,
+            2.0 * M_PI / a.ly, a.grp);
+        return cudaGetLastError();
+    }
+    if (!a.thomas && zmeet_modes(a.nz, sizeof(R)) > 0) return launch_zmeet<R>(a, s);
+    poisson_zsolve<R><<<dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s>>>(
+        (R2 *)a.spec, a.cpt, a.dpw, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz,
+        a.nxh, a.pitch, a.dz, a.eps, a.voltage, a.grp);
+    return cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t launch_poisson(const PoissonArgs &a, cudaStream_t s) {
-    using R2 = typename Cplx<R>::T;
     cudaError_t e;
     if (a.split && poisson_split_usable<R>(a)) {
         switch (a.ny / 64) {
@@ -2121,35 +2154,7 @@ cudaError_t launch_poisson(const PoissonArgs &a, cudaStream_t s) {
         return rows_inv<R>(a, s);
     }
     if ((e = cols<R, -1>(a, s)) != cudaSuccess) return e;
-    if (a.twz && poisson_fast_size(2 * (a.nz - 1))) {
-        switch (2 * (a.nz - 1)) {
-            case 48: e = zdst<R, 48>(a, s); break;
-            case 64: e = zdst<R, 64>(a, s); break;
-            case 80: e = zdst<R, 80>(a, s); break;
-            case 96: e = zdst<R, 96>(a, s); break;
-            case 128: e = zdst<R, 128>(a, s); break;
-            case 256: e = zdst<R, 256>(a, s); break;
-            default: e = zdst<R, 512>(a, s); break;
-        }
-        if (e != cudaSuccess) return e;
-    } else if (a.twz && !(a.thomas && a.cpt)) {
-        const int modes = a.nxh * a.ny;
-        const int L = 2 * (a.nz - 1);
-        const size_t sm = zdst_rt_smem(L, a.ztb, sizeof(R));
-        if ((e = set_smem(poisson_zdst_rt<R>, sm, s)) != cudaSuccess) return e;
-        const R2 *tw = (const R2 *)a.twz;
-        poisson_zdst_rt<R><<<dim3((modes + a.ztb - 1) / a.ztb, 1, a.ngrp), 256, sm, s>>>(
-            (R2 *)a.spec, tw, (const R *)(tw + L), a.pz, a.planesum, a.qmean, a.phi00, a.ez00,
-            a.nx, a.ny, a.nxh, a.pitch, a.ztb, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx,
-            2.0 * M_PI / a.ly, a.grp);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    } else {
-        const int modes = a.nxh * a.ny;
-        poisson_zsolve<R><<<dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s>>>(
-            (R2 *)a.spec, a.cpt, a.dpw, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz,
-            a.nxh, a.pitch, a.dz, a.eps, a.voltage, a.grp);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
+    if ((e = zsolve<R>(a, s)) != cudaSuccess) return e;
     if ((e = cols<R, 1>(a, s)) != cudaSuccess) return e;
     if ((e = rows_inv<R>(a, s)) != cudaSuccess) return e;
     return cudaSuccess;

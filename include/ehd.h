@@ -91,7 +91,8 @@ typedef struct ehd_tuning {
                                 applies, else the per-node kernel; 1: per-node */
     int32_t node_block_x;    /* per-node kernel block: x extent 16, 32, 64 or
                                 128, y extent 128 / node_block_x              */
-    int32_t fft_rows;        /* run-time-radix x FFT: rows per block          */
+    int32_t fft_rows;        /* run-time-radix x FFT (where it serves NX: see
+                                dft_usable, csrc/dft.cu): rows per block      */
     int32_t fft_cols;        /* run-time-radix y FFT: columns per block       */
     int32_t poisson_path;    /* 0: the split-y three-kernel Poisson solve
                                 where it applies (NX a power of two 64..512,
@@ -99,8 +100,9 @@ typedef struct ehd_tuning {
                                 else the five-kernel one; 1: five-kernel     */
     int32_t z_solve;         /* where 2 (NZ-1) is not a compile-time FFT
                                 size (48, 64, 80, 96, 128, 256, 512): 0 the
-                                sine transform with run-time FFT passes, 1 the
-                                FP64 Thomas sweep                             */
+                                two-sided Thomas solve in shared memory (where
+                                a column fits; BF16 storage: the sine transform
+                                with run-time passes), 1 the FP64 Thomas sweep */
     int32_t reserved[2];     /* must be 0                                     */
 } ehd_tuning;
 
