@@ -106,6 +106,7 @@ struct ehd_ctx {
     float2 *psum = nullptr;
     int psum_blocks = 0;   // psum slots per plane of the per-node kernel
     int rows_grid = 0;     // CTAs of the bulk-copy row kernel, 0: not available
+    bool pair = false;     // two nodes per thread (lbm_pair.cu) available
     ehd_tuning tune{};     // launch shapes (ehd_set_tuning)
     unsigned generation = 0;  // bumped by ehd_set_tuning
     int *err = nullptr;    // device flag set by a row-kernel wait that gave up
@@ -234,11 +235,22 @@ int lbm(ehd_ctx *c, bool macros) {
     a.psum = c->psum;
     a.err = c->err;
     const int loc = c->pops_local ? 1 : 0, ea = c->e_arrays ? 1 : 0;
-    const bool rows = c->rows_grid > 0 && c->tune.lbm_kernel == 0 && !loc && !ea;
+    const bool steady = c->tune.lbm_kernel == 0 && !loc && !ea;
+    const bool pair = c->pair && steady, rows = !pair && c->rows_grid > 0 && steady;
     a.rows_grid = rows ? c->rows_grid : 0;
     a.node_bx = c->tune.node_block_x;
     cudaError_t e = cudaErrorInvalidValue;
-    switch (c->prec) {
+    // psum slots: of plane 0, of the other planes
+    const int nrow = lbm_rows_slots_per_plane(c->p.nx, c->p.ny);
+    const int nblk0 = pair || rows ? nrow : c->psum_blocks;
+    const int nblk = pair ? lbm_pair_slots(c->p.nx, c->p.ny) : nblk0;
+    // (psum_blocks follows the node kernel's block shape, see ehd_set_tuning)
+    if (pair) {
+        e = c->prec == EHD_PREC_FP16 ? launch_lbm_plane0<__half, float>(a, c->sc, macros, c->stream)
+                                     : launch_lbm_plane0<Mix16, float>(a, c->sc, macros, c->stream);
+        if (e == cudaSuccess)
+            e = launch_lbm_pair(c->prec, a, c->sc, macros, c->psum + nblk0, c->stream);
+    } else switch (c->prec) {
         case EHD_PREC_FP64: e = launch_lbm_step<double, double>(a, c->sc, loc, ea, macros, c->stream); break;
         case EHD_PREC_FP32: e = launch_lbm_step<float, float>(a, c->sc, loc, ea, macros, c->stream); break;
         case EHD_PREC_FP16: e = launch_lbm_step<__half, float>(a, c->sc, loc, ea, macros, c->stream); break;
@@ -250,11 +262,9 @@ int lbm(ehd_ctx *c, bool macros) {
     // buffer p will next be written against the means of the state it holds
     // now (the same phase of the injector's two-step alternation)
     const int p = c->cur;
-    const int nblk = rows ? lbm_rows_slots_per_plane(c->p.nx, c->p.ny) : c->psum_blocks;
-    // (psum_blocks follows the node kernel's block shape, see ehd_set_tuning)
     e = c->rsize == 8
-            ? launch_reduce_tables<double>(c->psum, c->mean[p ^ 1], nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream)
-            : launch_reduce_tables<float>(c->psum, c->mean[p ^ 1], nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream);
+            ? launch_reduce_tables<double>(c->psum, c->mean[p ^ 1], nblk0, nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream)
+            : launch_reduce_tables<float>(c->psum, c->mean[p ^ 1], nblk0, nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream);
     if (e != cudaSuccess) return fail(EHD_ERR_CUDA, "reference tables: %s", cudaGetErrorString(e));
     c->cur ^= 1;
     c->pops_local = false;
@@ -470,6 +480,7 @@ int ctx_step_args(ehd_ctx *c, bool macros, LbmArgs *la, StepConst *sc, ReduceDes
     rd->nxy = c->sc.nxy;
     rd->nblk = rows ? lbm_rows_slots_per_plane(c->p.nx, c->p.ny)
                     : lbm_blocks_per_plane(c->p.nx, c->p.ny, c->tune.node_block_x);
+    rd->nblk0 = rd->nblk;
     rd->nz = c->p.nz;
     // poisson() after lbm() reads the plane means of the new state
     *pa = c->pa;
@@ -592,7 +603,9 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     }
     {
         // room for the plane sums of every launch shape ehd_set_tuning allows
-        int slots = c->rows_grid > 0 ? lbm_rows_slots_per_plane(nx, ny) : 0;
+        c->pair = lbm_pair_usable(nx, c->sc.n, c->prec);
+        int slots = c->rows_grid > 0 || c->pair ? lbm_rows_slots_per_plane(nx, ny) : 0;
+        if (c->pair) slots = std::max(slots, lbm_pair_slots(nx, ny));
         for (int bx = 16; bx <= 128; bx *= 2) slots = std::max(slots, lbm_blocks_per_plane(nx, ny, bx));
         if ((r = dalloc(c, (void **)&c->psum, sizeof(float2) * (size_t)slots * nz))) return bail(r);
     }

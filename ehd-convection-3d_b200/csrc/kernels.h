@@ -22,6 +22,19 @@ struct LbmArgs {
     int node_bx;                    // per-node kernel block: node_bx x (128 / node_bx)
 };
 
+// ---- two nodes per thread, FP16 flow populations (csrc/lbm_pair.cu) ----
+// whether it serves a grid of n nodes (prec: ehd_precision); psum slots of a
+// plane z >= 1 (those of z = 0 come first, lbm_rows_slots_per_plane of them)
+bool lbm_pair_usable(int nx, long long n, int prec);
+int lbm_pair_slots(int nx, int ny);
+// planes z >= 1 of a steady-state step, plane sums from psum on
+cudaError_t launch_lbm_pair(int prec, const LbmArgs &a, const StepConst &c, bool macros,
+                            float2 *psum, cudaStream_t s);
+// plane z = 0 of a steady-state step on the per-node kernel, its plane sums in
+// lbm_rows_slots_per_plane slots
+template <typename T, typename R>
+cudaError_t launch_lbm_plane0(const LbmArgs &a, const StepConst &c, bool macros, cudaStream_t s);
+
 template <typename T, typename R>
 cudaError_t launch_lbm_step(const LbmArgs &a, const StepConst &c, int local_pops, int e_arrays,
                             bool macros, cudaStream_t s);
@@ -53,10 +66,11 @@ template <typename R>
 cudaError_t launch_build_tables(const double *msrc, double *wdst, const double *wread,
                                 void *ktab, const StepConst &c, cudaStream_t s);
 // psum_reduce and build_tables in one launch (the tables read msrc, the
-// previous means, so the two parts are independent)
+// previous means, so the two parts are independent); nblk0 slots of plane 0,
+// then nblk of each other plane
 template <typename R>
-cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk, const double *msrc,
-                                 double *wdst, const double *wread, void *ktab,
+cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk0, int nblk,
+                                 const double *msrc, double *wdst, const double *wread, void *ktab,
                                  const StepConst &c, cudaStream_t s);
 // ---- launches over a group of instances with the same grid ----------------
 // (batch steps, csrc/batch.cu): one launch per kernel covers every instance.
@@ -84,7 +98,7 @@ struct ReduceDesc {
     const double *wread;
     void *ktab;
     long long nxy;
-    int nblk, nz;
+    int nblk0, nblk, nz;
 };
 template <typename R>
 cudaError_t launch_reduce_tables_group(const ReduceDesc *desc_dev, int n, int nz, cudaStream_t s);

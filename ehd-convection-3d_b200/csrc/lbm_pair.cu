@@ -1,0 +1,342 @@
+// lbm_pair.cu -- the steady-state step with two nodes per thread, for FP16
+// flow populations (FP16 and mixed storage) on grids of even NX.
+//
+// With 2-byte populations the one-node-per-thread kernel is bound by the
+// issue of its instructions, not by memory: about 1,400 a node, at 512 x 512 x
+// 129 2.23 ms against 1.17 ms for its bytes at the copy bandwidth.  Here a
+// thread owns the nodes x and x + 1 of a row (x even), and every operation
+// from the loads to the stores is one instruction for both: a population pair
+// is one 32-bit word (two, for the directions with e_x != 0, whose halves are
+// put together by a byte permute), the arithmetic runs on packed FP32x2
+// values, one per node, and a result pair is one conversion and one 32-bit
+// store.  Planes are walked as runs of node pairs, so that no lane is idle at
+// the end of a row.  That is 860 instructions a node; with the 168 registers
+// of three blocks a multiprocessor (12 warps) the step of 512 x 512 x 129 in
+// FP16 went 2.82 -> 2.15 ms (this kernel 1.65 ms; with two or four blocks,
+// 255 or 128 registers, 2.62 and 2.66 ms), 256 x 256 x 129 in mixed storage
+// 0.690 -> 0.598 ms (there against the row kernel), 302 x 266 x 38 mixed 333 ->
+// 227 us for the LBM half.  What is left to the floor is load latency at that
+// occupancy (2.3 of 5.7 cycles between issues).
+//
+// The injector plane z = 0 stays on the one-node kernel in a launch of its
+// own.  The pull, collision and wall rules are those of lbm.cu (finish_node),
+// on the same deviations.
+#include <type_traits>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace ehd {
+
+namespace {
+
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+
+// e_d . (a, b, c), the components of e_d in {-1, 0, 1}; m = (-1, -1)
+__device__ __forceinline__ float2 dot2(int d, float2 a, float2 b, float2 c, float2 m) {
+    float2 s = make_float2(0.f, 0.f);
+    bool any = false;
+    const int e[3] = {ex_of(d), ey_of(d), ez_of(d)};
+    const float2 v[3] = {a, b, c};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if (e[i] == 0) continue;
+        if (!any) s = e[i] > 0 ? v[i] : neg2(v[i]);
+        else s = e[i] > 0 ? add2(s, v[i]) : fma2(m, v[i], s);
+        any = true;
+    }
+    return s;
+}
+
+// The pair (x + c, x + c + 1) of a direction's row, c = -e_x: from byte
+// offsets of the words holding x - 2, x and x + 2 (wrapped in the row).
+__device__ __forceinline__ float2 pull(const __half *p, unsigned om, unsigned o0, unsigned op, int ex) {
+    const char *b = reinterpret_cast<const char *>(p);
+    unsigned w = __ldg(reinterpret_cast<const unsigned *>(b + o0));
+    if (ex > 0) w = __byte_perm(__ldg(reinterpret_cast<const unsigned *>(b + om)), w, 0x5432);
+    if (ex < 0) w = __byte_perm(w, __ldg(reinterpret_cast<const unsigned *>(b + op)), 0x5432);
+    return __half22float2(*reinterpret_cast<const __half2 *>(&w));
+}
+// the same for FP32 rows: twice the byte offsets
+__device__ __forceinline__ float2 pull(const float *p, unsigned om, unsigned o0, unsigned op, int ex) {
+    const char *b = reinterpret_cast<const char *>(p);
+    if (ex == 0) return __ldg(reinterpret_cast<const float2 *>(b + 2 * o0));
+    const float *q = reinterpret_cast<const float *>(b + 2 * o0);
+    if (ex > 0) return make_float2(__ldg(reinterpret_cast<const float *>(b + 2 * om) + 1), __ldg(q));
+    return make_float2(__ldg(q + 1), __ldg(reinterpret_cast<const float *>(b + 2 * op)));
+}
+__device__ __forceinline__ void put(__half *p, unsigned o, float2 v) {
+    *reinterpret_cast<__half2 *>(reinterpret_cast<char *>(p) + o) = __float22half2_rn(v);
+}
+__device__ __forceinline__ void put(float *p, unsigned o, float2 v) {
+    *reinterpret_cast<float2 *>(reinterpret_cast<char *>(p) + 2 * o) = v;
+}
+
+constexpr int kPairThreads = 128;
+
+}  // namespace
+
+template <typename T>
+struct PairArgs {
+    PopPtrs<T> pp;
+    const float *phip;
+    const double *ez00;
+    float *qout, *rout, *uout, *vout, *wout;
+    const float *zref;
+    float2 *psum;  // slots of the planes z >= 1: [z - 1][warp]
+};
+
+template <typename T, bool MACROS>
+__global__ void __launch_bounds__(kPairThreads, 3)
+lbm_pair_kernel(const PairArgs<T> a, const KConst<float> c) {
+    const int NX = c.nx, NY = c.ny, NZ = c.nz, hx = NX / 2;
+    const int z = 1 + blockIdx.y;
+    const int pairs = hx * NY;
+    const int i = blockIdx.x * kPairThreads + threadIdx.x;
+    // lanes past the plane work on its last pair (the whole warp takes part in
+    // the plane sums) and store nothing
+    const bool inside = i < pairs;
+    const int ic = inside ? i : pairs - 1;
+    const int y = ic / hx, xp2 = ic - y * hx;  // pair of the row
+    const int ym = y == 0 ? NY - 1 : y - 1, yp = y == NY - 1 ? 0 : y + 1;
+    const int zm = z - 1, zp = z == NZ - 1 ? 0 : z + 1;
+    // byte offsets of 2-byte elements: word of the pair, of the pair before
+    // and after it in the row
+    const unsigned x0 = 4u * xp2, xm = xp2 == 0 ? 4u * (hx - 1) : x0 - 4u,
+                   xq = xp2 == hx - 1 ? 0u : x0 + 4u;
+    unsigned row[3][3];  // [e_y + 1][e_z + 1]: byte offset of row (y - e_y, z - e_z)
+    {
+        const int ys[3] = {yp, y, ym}, zs[3] = {zp, z, zm};
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+                row[u][v] = 2u * (unsigned)NX * ((unsigned)ys[u] + (unsigned)NY * (unsigned)zs[v]);
+    }
+    float zr[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) zr[k] = __ldg(a.zref + 10 * z + k);
+    const float2 mone = dup(-1.f), half = dup(0.5f);
+
+    // ---- pull and moments ----
+    float2 f[Q], h[Q];
+    float2 drho = dup(0.f), dq = dup(0.f), mx = dup(0.f), my = dup(0.f), mz = dup(0.f);
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+        const unsigned r = row[ey_of(d) + 1][ez_of(d) + 1];
+        f[d] = pull(a.pp.fa[d], r + xm, r + x0, r + xq, ex_of(d));
+        h[d] = pull(a.pp.ha[d], r + xm, r + x0, r + xq, ex_of(d));
+    }
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+        const float w = c.w[cls_of(d)];
+        f[d] = add2(f[d], dup(w * (ez_of(d) > 0 ? zr[2] : (ez_of(d) < 0 ? zr[4] : zr[3]))));
+        h[d] = add2(h[d], dup(w * (ez_of(d) > 0 ? zr[5] : (ez_of(d) < 0 ? zr[7] : zr[6]))));
+        drho = add2(drho, f[d]);
+        dq = add2(dq, h[d]);
+        if (ex_of(d)) mx = ex_of(d) > 0 ? add2(mx, f[d]) : fma2(mone, f[d], mx);
+        if (ey_of(d)) my = ey_of(d) > 0 ? add2(my, f[d]) : fma2(mone, f[d], my);
+        if (ez_of(d)) mz = ez_of(d) > 0 ? add2(mz, f[d]) : fma2(mone, f[d], mz);
+    }
+    const float2 rho = add2(dup(zr[0]), drho), charge = add2(dup(zr[1]), dq);
+    {
+        float2 v = make_float2(inside ? rho.x + rho.y : 0.f, inside ? charge.x + charge.y : 0.f);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        if ((threadIdx.x & 31) == 0)
+            a.psum[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (kPairThreads / 32) +
+                   (threadIdx.x >> 5)] = v;
+    }
+    if (!inside) return;
+
+    // ---- E = -grad(phi), central differences (see finish_node) ----
+    const unsigned node = row[1][1] / 2u + 2u * xp2;  // of the pair's first node
+    float2 Ex, Ey, Ez;
+    {
+        auto pair_at = [&](unsigned o) { return __ldg(reinterpret_cast<const float2 *>(a.phip + o)); };
+        const unsigned r = row[1][1] / 2u;
+        const float2 p0 = pair_at(r + 2u * xp2);
+        const float pm = __ldg(a.phip + r + xm / 2u + 1u), pp = __ldg(a.phip + r + xq / 2u);
+        Ex = mul2(fma2(mone, make_float2(p0.y, pp), make_float2(pm, p0.x)), dup(c.inv2dx));
+        // row[][1]: e_y = +1 is the row y - 1
+        Ey = mul2(fma2(mone, pair_at(row[0][1] / 2u + 2u * xp2), pair_at(row[2][1] / 2u + 2u * xp2)),
+                  dup(c.inv2dy));
+        const int zc = z > NZ - 2 ? NZ - 2 : z;
+        const unsigned nc = node - (unsigned)(z - zc) * c.nxy;
+        Ez = fma2(fma2(mone, pair_at(nc + c.nxy), pair_at(nc - c.nxy)), dup(c.inv2dz),
+                  dup((float)__ldg(a.ez00 + zc)));
+    }
+    const float2 fx = fma2(charge, Ex, dup(c.exf)), fy = mul2(charge, Ey), fz = mul2(charge, Ez);
+    const float2 rinv = make_float2(1.f / rho.x, 1.f / rho.y);
+    const float2 ci = dup(c.cflinv), dh = dup(c.dt_half);
+    const float2 ux = mul2(rinv, fma2(mx, ci, mul2(fx, dh)));
+    const float2 uy = mul2(rinv, fma2(my, ci, mul2(fy, dh)));
+    const float2 uz = mul2(rinv, fma2(mz, ci, mul2(fz, dh)));
+    *reinterpret_cast<float2 *>(a.qout + node) = charge;
+    if (MACROS) {
+        *reinterpret_cast<float2 *>(a.rout + node) = rho;
+        *reinterpret_cast<float2 *>(a.uout + node) = ux;
+        *reinterpret_cast<float2 *>(a.vout + node) = uy;
+        *reinterpret_cast<float2 *>(a.wout + node) = uz;
+    }
+    const unsigned o = 2u * node;  // byte offset of 2-byte elements
+
+    // ---- f: collision, or the wall rule of the collector plane ----
+    if (z == NZ - 1) {
+        put(a.pp.fb[0], o, f[0]);
+#pragma unroll
+        for (int d = 1; d < Q; ++d) {
+            float2 v = f[opp_of(d)];
+            if (mw_sign_of(d) != 0) v = add2(v, dup(c.mw[d]));
+            put(a.pp.fb[d], o, v);
+        }
+        return;  // its g is written by the plane below
+    }
+    {
+        const float2 usq = mul2(fma2(ux, ux, fma2(uy, uy, mul2(uz, uz))), dup(0.5f * c.inv_cs2));
+        const float2 t = dup(c.inv_cs2cfl);
+        const float2 tux = mul2(ux, t), tuy = mul2(uy, t), tuz = mul2(uz, t);
+        const float2 uF = fma2(ux, fx, fma2(uy, fy, mul2(uz, fz)));
+        const float2 rp_hi = dup(c.rate_hi[0]), nrp_lo = dup(-c.rate_lo[0]);
+        const float2 rm_hi = dup(c.rate_hi[1]), nrm_lo = dup(-c.rate_lo[1]);
+        float2 nWR[4], PK[4], QK[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            nWR[k] = mul2(dup(-c.w[k]), rho);
+            PK[k] = fma2(neg2(nWR[k]), usq, mul2(dup(-c.w[k]), drho));
+            QK[k] = mul2(dup(c.c3[k]), uF);
+        }
+        {
+            const float2 X = add2(f[0], PK[0]);
+            const float2 A = fma2(rp_hi, X, fma2(nrp_lo, X, QK[0]));
+            put(a.pp.fb[0], o, fma2(mone, A, f[0]));
+        }
+#pragma unroll
+        for (int d = 1; d < Q; d += 2) {
+            const int k = cls_of(d);
+            const float2 fd = f[d], fo = f[d + 1];
+            const float2 cu = dot2(d, tux, tuy, tuz, mone), eF = dot2(d, fx, fy, fz, mone);
+            const float2 wc = mul2(nWR[k], cu);
+            float2 X = fma2(half, add2(fd, fo), PK[k]);
+            X = fma2(mul2(half, wc), cu, X);
+            float2 A = fma2(nrp_lo, X, QK[k]);
+            A = fma2(rp_hi, X, A);
+            A = fma2(dup(-c.c1[k]), mul2(cu, eF), A);
+            const float2 Y = fma2(half, fma2(mone, fo, fd), wc);
+            float2 B = fma2(nrm_lo, Y, mul2(dup(-c.c2[k]), eF));
+            B = fma2(rm_hi, Y, B);
+            put(a.pp.fb[d], o, fma2(mone, add2(A, B), fd));
+            put(a.pp.fb[d + 1], o, fma2(mone, A, add2(fo, B)));
+        }
+    }
+
+    // ---- g: collision; the plane below the collector writes the collector's
+    // copy too, relative to its reference ----
+    {
+        const float2 Kd = dup(c.K);
+        const float2 ucx = fma2(Kd, Ex, ux), ucy = fma2(Kd, Ey, uy), ucz = fma2(Kd, Ez, uz);
+        const float2 usq = mul2(fma2(ucx, ucx, fma2(ucy, ucy, mul2(ucz, ucz))), dup(0.5f * c.inv_cs2));
+        const float2 t = dup(c.inv_cs2cfl);
+        const float2 tux = mul2(ucx, t), tuy = mul2(ucy, t), tuz = mul2(ucz, t);
+        const float2 cp_hi = dup(c.rate_hi[2]), ncp_lo = dup(-c.rate_lo[2]);
+        const float2 cm_hi = dup(c.rate_hi[3]), cm_lo = dup(c.rate_lo[3]);
+        const bool over = c.rate_hi[3] == 2.f, top = z == NZ - 2;
+        const unsigned ou = o + 2u * c.nxy;
+        float2 nWQ[4], PQ[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            nWQ[k] = mul2(dup(-c.w[k]), charge);
+            PQ[k] = fma2(neg2(nWQ[k]), usq, mul2(dup(-c.w[k]), dq));
+        }
+        {
+            const float2 X = add2(h[0], PQ[0]);
+            const float2 A = fma2(cp_hi, X, mul2(ncp_lo, X));
+            const float2 out = fma2(mone, A, h[0]);
+            put(a.pp.hb[0], o, out);
+            if (top) put(a.pp.hb[0], ou, add2(out, dup(c.w[0] * zr[8])));
+        }
+#pragma unroll
+        for (int d = 1; d < Q; d += 2) {
+            const int k = cls_of(d);
+            const float2 hd = h[d], ho = h[d + 1];
+            const float2 cu = dot2(d, tux, tuy, tuz, mone);
+            const float2 wc = mul2(nWQ[k], cu);
+            float2 X = fma2(half, add2(hd, ho), PQ[k]);
+            X = fma2(mul2(half, wc), cu, X);
+            const float2 A = fma2(cp_hi, X, mul2(ncp_lo, X));
+            const float2 Y = fma2(half, fma2(mone, ho, hd), wc);
+            float2 od, oo;
+            if (over) {
+                // hd - B and ho + B without forming them (see g_pair2)
+                const float2 t2 = add2(wc, wc);  // -2 WQ cu
+                od = fma2(cm_lo, Y, fma2(mone, A, fma2(mone, t2, ho)));
+                oo = fma2(neg2(cm_lo), Y, fma2(mone, A, add2(hd, t2)));
+            } else {
+                const float2 B = fma2(cm_hi, Y, mul2(neg2(cm_lo), Y));
+                od = fma2(mone, add2(A, B), hd);
+                oo = fma2(mone, A, add2(ho, B));
+            }
+            put(a.pp.hb[d], o, od);
+            put(a.pp.hb[d + 1], o, oo);
+            if (top) {
+                const float2 up = dup(c.w[k] * zr[8]);
+                put(a.pp.hb[d], ou, add2(od, up));
+                put(a.pp.hb[d + 1], ou, add2(oo, up));
+            }
+        }
+    }
+}
+
+// psum slots of a plane z >= 1
+int lbm_pair_slots(int nx, int ny) {
+    const int pairs = nx / 2 * ny;
+    return (pairs + kPairThreads - 1) / kPairThreads * (kPairThreads / 32);
+}
+
+// FP16 f with FP16 or FP32 g, rows of whole pairs, 32-bit byte offsets of the
+// 4-byte arrays
+bool lbm_pair_usable(int nx, long long n, int prec) {
+    return (prec == 2 || prec == 4) && nx % 2 == 0 && n < (1LL << 30);
+}
+
+template <typename T>
+static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macros, float2 *psum,
+                               cudaStream_t s) {
+    PairArgs<T> a;
+    for (int d = 0; d < Q; ++d) {
+        a.pp.fa[d] = (const typename PopT<T>::F *)la.fa + (size_t)d * c.n;
+        a.pp.ha[d] = (const typename PopT<T>::G *)la.ha + (size_t)d * c.n;
+        a.pp.fb[d] = (typename PopT<T>::F *)la.fb + (size_t)d * c.n;
+        a.pp.hb[d] = (typename PopT<T>::G *)la.hb + (size_t)d * c.n;
+    }
+    a.phip = (const float *)la.phip;
+    a.ez00 = la.ez00;
+    a.qout = (float *)la.q;
+    a.rout = (float *)la.rho;
+    a.uout = (float *)la.u;
+    a.vout = (float *)la.v;
+    a.wout = (float *)la.w;
+    a.zref = (const float *)la.zref;
+    a.psum = psum;
+    const KConst<float> k = make_kconst<float>(c);
+    const int pairs = c.nx / 2 * c.ny;
+    const dim3 grid((pairs + kPairThreads - 1) / kPairThreads, c.nz - 1);
+    if (macros) lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(a, k);
+    else lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(a, k);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lbm_pair(int prec, const LbmArgs &la, const StepConst &c, bool macros,
+                            float2 *psum, cudaStream_t s) {
+    return prec == 2 ? pair_launch<__half>(la, c, macros, psum, s)
+                     : pair_launch<Mix16>(la, c, macros, psum, s);
+}
+
+}  // namespace ehd

@@ -87,8 +87,10 @@ typedef struct ehd_ctx ehd_ctx;
  * shape changes only the order of the FP32 partial plane sums behind the
  * per-plane reference states, i.e. results at round-off level. */
 typedef struct ehd_tuning {
-    int32_t lbm_kernel;      /* 0: steady steps on the row kernel where it
-                                applies, else the per-node kernel; 1: per-node */
+    int32_t lbm_kernel;      /* 0: steady steps on the kernel made for the grid
+                                and storage (columns; node pairs, FP16 f; rows)
+                                where one applies, else the per-node kernel;
+                                1: per-node                                   */
     int32_t node_block_x;    /* per-node kernel block: x extent 16, 32, 64 or
                                 128, y extent 128 / node_block_x              */
     int32_t fft_rows;        /* run-time-radix x FFT (where it serves NX: see
