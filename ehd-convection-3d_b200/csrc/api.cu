@@ -241,15 +241,12 @@ int lbm(ehd_ctx *c, bool macros) {
     a.node_bx = c->tune.node_block_x;
     cudaError_t e = cudaErrorInvalidValue;
     // psum slots: of plane 0, of the other planes
-    const int nrow = lbm_rows_slots_per_plane(c->p.nx, c->p.ny);
-    const int nblk0 = pair || rows ? nrow : c->psum_blocks;
-    const int nblk = pair ? lbm_pair_slots(c->p.nx, c->p.ny) : nblk0;
+    const int nblk = pair ? lbm_pair_slots(c->p.nx, c->p.ny)
+                          : (rows ? lbm_rows_slots_per_plane(c->p.nx, c->p.ny) : c->psum_blocks);
+    const int nblk0 = pair ? 2 * nblk : nblk;
     // (psum_blocks follows the node kernel's block shape, see ehd_set_tuning)
     if (pair) {
-        e = c->prec == EHD_PREC_FP16 ? launch_lbm_plane0<__half, float>(a, c->sc, macros, c->stream)
-                                     : launch_lbm_plane0<Mix16, float>(a, c->sc, macros, c->stream);
-        if (e == cudaSuccess)
-            e = launch_lbm_pair(c->prec, a, c->sc, macros, c->psum + nblk0, c->stream);
+        e = launch_lbm_pair(c->prec, a, c->sc, macros, c->stream);
     } else switch (c->prec) {
         case EHD_PREC_FP64: e = launch_lbm_step<double, double>(a, c->sc, loc, ea, macros, c->stream); break;
         case EHD_PREC_FP32: e = launch_lbm_step<float, float>(a, c->sc, loc, ea, macros, c->stream); break;
@@ -604,8 +601,8 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     {
         // room for the plane sums of every launch shape ehd_set_tuning allows
         c->pair = lbm_pair_usable(nx, c->sc.n, c->prec);
-        int slots = c->rows_grid > 0 || c->pair ? lbm_rows_slots_per_plane(nx, ny) : 0;
-        if (c->pair) slots = std::max(slots, lbm_pair_slots(nx, ny));
+        int slots = c->rows_grid > 0 ? lbm_rows_slots_per_plane(nx, ny) : 0;
+        if (c->pair) slots = std::max(slots, 2 * lbm_pair_slots(nx, ny));
         for (int bx = 16; bx <= 128; bx *= 2) slots = std::max(slots, lbm_blocks_per_plane(nx, ny, bx));
         if ((r = dalloc(c, (void **)&c->psum, sizeof(float2) * (size_t)slots * nz))) return bail(r);
     }

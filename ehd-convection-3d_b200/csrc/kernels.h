@@ -24,16 +24,11 @@ struct LbmArgs {
 
 // ---- two nodes per thread, FP16 flow populations (csrc/lbm_pair.cu) ----
 // whether it serves a grid of n nodes (prec: ehd_precision); psum slots of a
-// plane z >= 1 (those of z = 0 come first, lbm_rows_slots_per_plane of them)
+// plane z >= 1 (those of z = 0, twice as many, come first)
 bool lbm_pair_usable(int nx, long long n, int prec);
 int lbm_pair_slots(int nx, int ny);
-// planes z >= 1 of a steady-state step, plane sums from psum on
 cudaError_t launch_lbm_pair(int prec, const LbmArgs &a, const StepConst &c, bool macros,
-                            float2 *psum, cudaStream_t s);
-// plane z = 0 of a steady-state step on the per-node kernel, its plane sums in
-// lbm_rows_slots_per_plane slots
-template <typename T, typename R>
-cudaError_t launch_lbm_plane0(const LbmArgs &a, const StepConst &c, bool macros, cudaStream_t s);
+                            cudaStream_t s);
 
 template <typename T, typename R>
 cudaError_t launch_lbm_step(const LbmArgs &a, const StepConst &c, int local_pops, int e_arrays,

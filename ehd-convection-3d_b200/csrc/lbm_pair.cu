@@ -18,13 +18,16 @@
 // 227 us for the LBM half.  What is left to the floor is load latency at that
 // occupancy (2.3 of 5.7 cycles between issues).
 //
-// The injector plane z = 0 stays on the one-node kernel in a launch of its
-// own.  The pull, collision and wall rules are those of lbm.cu (finish_node),
-// on the same deviations.
+// The injector plane z = 0 is stepped with one node per thread (node_step), by
+// blocks of the same launch on small grids, in a launch of its own on large
+// ones.  The pull, collision and wall rules are those of finish_node, on the
+// same deviations.  (Rows through shared memory, as in lbm_rows_kernel, with
+// g read twice to stay at 128 registers, took 2.53 ms where this takes 2.15.)
 #include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
+#include "lbm_node.cuh"
 
 namespace ehd {
 
@@ -90,12 +93,38 @@ struct PairArgs {
     float2 *psum;  // slots of the planes z >= 1: [z - 1][warp]
 };
 
+// Block b of plane 0, one node per thread; its plane sums come first.
 template <typename T, bool MACROS>
+__device__ __forceinline__ void plane0_block(const StepArgs<T, float> &a, const KConst<float> &c,
+                                             int b) {
+    const int i = b * kPairThreads + threadIdx.x;
+    const bool in = i < c.nx * c.ny;
+    const int y = in ? i / c.nx : c.ny - 1, x = in ? i - y * c.nx : c.nx - 1;
+    node_step<T, float, MACROS>(
+        a, c, x, y, 0, in, [&] { return b * (kPairThreads / 32) + (threadIdx.x >> 5); }, false,
+        false);
+}
+template <typename T, bool MACROS>
+__global__ void __launch_bounds__(kPairThreads, 4)
+lbm_plane0_kernel(const StepArgs<T, float> a, const KConst<float> c) {
+    plane0_block<T, MACROS>(a, c, blockIdx.x);
+}
+
+// Planes z >= 1 (Args = PairArgs), or plane 0 as well (Args = StepArgs), as
+// blockIdx.y = 0, 1 with twice as many blocks as a plane of pairs.
+template <typename T, bool MACROS, typename Args>
 __global__ void __launch_bounds__(kPairThreads, 3)
-lbm_pair_kernel(const PairArgs<T> a, const KConst<float> c) {
+lbm_pair_kernel(const Args a, const KConst<float> c) {
+    constexpr bool kPlane0 = std::is_same<Args, StepArgs<T, float>>::value;
     const int NX = c.nx, NY = c.ny, NZ = c.nz, hx = NX / 2;
-    const int z = 1 + blockIdx.y;
     const int pairs = hx * NY;
+    if constexpr (kPlane0) {
+        if (blockIdx.y < 2) {
+            plane0_block<T, MACROS>(a, c, 2 * blockIdx.x + blockIdx.y);
+            return;
+        }
+    }
+    const int z = kPlane0 ? (int)blockIdx.y - 1 : 1 + (int)blockIdx.y;
     const int i = blockIdx.x * kPairThreads + threadIdx.x;
     // lanes past the plane work on its last pair (the whole warp takes part in
     // the plane sums) and store nothing
@@ -294,7 +323,7 @@ lbm_pair_kernel(const PairArgs<T> a, const KConst<float> c) {
     }
 }
 
-// psum slots of a plane z >= 1
+// psum slots of a plane z >= 1 (plane 0: twice as many)
 int lbm_pair_slots(int nx, int ny) {
     const int pairs = nx / 2 * ny;
     return (pairs + kPairThreads - 1) / kPairThreads * (kPairThreads / 32);
@@ -306,37 +335,49 @@ bool lbm_pair_usable(int nx, long long n, int prec) {
     return (prec == 2 || prec == 4) && nx % 2 == 0 && n < (1LL << 30);
 }
 
+// Up to so many blocks of pairs plane 0 goes with them: 64 x 64 x 33 in FP16
+// (512 blocks) 30.7 us a step with a launch of its own, 25.6 without, 100 x
+// 100 x 50 (2,000) 79.7 and 72.9; with many blocks the launch is nothing and the
+// kernel without the extra branch is the faster one: 256 x 256 x 129 (32,768)
+// 498 and 535.
+constexpr long long kMergeBlocks = 5000;
+
 template <typename T>
-static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macros, float2 *psum,
-                               cudaStream_t s) {
-    PairArgs<T> a;
-    for (int d = 0; d < Q; ++d) {
-        a.pp.fa[d] = (const typename PopT<T>::F *)la.fa + (size_t)d * c.n;
-        a.pp.ha[d] = (const typename PopT<T>::G *)la.ha + (size_t)d * c.n;
-        a.pp.fb[d] = (typename PopT<T>::F *)la.fb + (size_t)d * c.n;
-        a.pp.hb[d] = (typename PopT<T>::G *)la.hb + (size_t)d * c.n;
-    }
-    a.phip = (const float *)la.phip;
-    a.ez00 = la.ez00;
-    a.qout = (float *)la.q;
-    a.rout = (float *)la.rho;
-    a.uout = (float *)la.u;
-    a.vout = (float *)la.v;
-    a.wout = (float *)la.w;
-    a.zref = (const float *)la.zref;
-    a.psum = psum;
+static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macros, cudaStream_t s) {
+    const StepArgs<T, float> a = make_step_args<T, float>(la, c);
     const KConst<float> k = make_kconst<float>(c);
-    const int pairs = c.nx / 2 * c.ny;
-    const dim3 grid((pairs + kPairThreads - 1) / kPairThreads, c.nz - 1);
-    if (macros) lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(a, k);
-    else lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(a, k);
+    const int pairs = c.nx / 2 * c.ny, nb = (pairs + kPairThreads - 1) / kPairThreads;
+    if (nb * (long long)(c.nz - 1) <= kMergeBlocks) {
+        const dim3 grid(nb, c.nz + 1);
+        if (macros) lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(a, k);
+        else lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(a, k);
+        return cudaGetLastError();
+    }
+    PairArgs<T> p;
+    p.pp = a.pp;
+    p.phip = a.phip;
+    p.ez00 = a.ez00;
+    p.qout = a.qout;
+    p.rout = a.rout;
+    p.uout = a.uout;
+    p.vout = a.vout;
+    p.wout = a.wout;
+    p.zref = a.zref;
+    p.psum = a.psum + 2 * lbm_pair_slots(c.nx, c.ny);
+    const dim3 grid(nb, c.nz - 1);
+    if (macros) {
+        lbm_plane0_kernel<T, true><<<2 * nb, kPairThreads, 0, s>>>(a, k);
+        lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(p, k);
+    } else {
+        lbm_plane0_kernel<T, false><<<2 * nb, kPairThreads, 0, s>>>(a, k);
+        lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(p, k);
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_lbm_pair(int prec, const LbmArgs &la, const StepConst &c, bool macros,
-                            float2 *psum, cudaStream_t s) {
-    return prec == 2 ? pair_launch<__half>(la, c, macros, psum, s)
-                     : pair_launch<Mix16>(la, c, macros, psum, s);
+                            cudaStream_t s) {
+    return prec == 2 ? pair_launch<__half>(la, c, macros, s) : pair_launch<Mix16>(la, c, macros, s);
 }
 
 }  // namespace ehd
