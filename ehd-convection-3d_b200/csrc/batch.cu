@@ -248,7 +248,7 @@ int step_graph(ehd_batch *b, const std::vector<char> &act, bool macros, cudaGrap
             r = cuda_fail("batch fork wait", e);
             break;
         }
-        if ((r = ctx_launch_step(c, macros)) != EHD_OK) break;
+        if ((r = ctx_capture_steps(c, 1, macros)) != EHD_OK) break;
         if ((e = cudaEventRecord(b->join[i], ctx_stream(c))) != cudaSuccess ||
             (e = cudaStreamWaitEvent(b->stream, b->join[i], 0)) != cudaSuccess)
             r = cuda_fail("batch join", e);
@@ -298,7 +298,7 @@ int graph_steps(ehd_batch *b, const std::vector<char> &act, int k, int nsteps) {
             break;
         }
         for (size_t i = 0; i < b->inst.size(); ++i)
-            if (act[i]) ctx_commit_step(b->inst[i]);
+            if (act[i]) ctx_commit_steps(b->inst[i], 1);
     }
     const int r2 = order(b, act, false);
     return r != EHD_OK ? r : r2;

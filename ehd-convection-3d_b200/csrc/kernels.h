@@ -255,9 +255,8 @@ double *ctx_time(::ehd_ctx *c);
 
 // For the batch (csrc/batch.cu): a context's stream, device and precision;
 // whether its next step can be captured (not the first after an upload);
-// its buffer parity; the launches of one steady step on its stream with the
-// buffer parity left unchanged (as a graph capture needs); and the
-// bookkeeping once that step has run.
+// its buffer parity; steady steps into a capture on its stream, with the buffer
+// parity left unchanged; and the bookkeeping once they have run.
 cudaStream_t ctx_stream(const ::ehd_ctx *c);
 int ctx_device(const ::ehd_ctx *c);
 int ctx_precision(const ::ehd_ctx *c);
@@ -266,8 +265,8 @@ bool ctx_steady(const ::ehd_ctx *c);
 // of them at once, so a batch leaves such an instance to its own stream)
 bool ctx_column(const ::ehd_ctx *c);
 int ctx_parity(const ::ehd_ctx *c);
-int ctx_launch_step(::ehd_ctx *c, bool macros);
-void ctx_commit_step(::ehd_ctx *c);
+int ctx_capture_steps(::ehd_ctx *c, int steps, bool macros);
+void ctx_commit_steps(::ehd_ctx *c, int steps);
 // changes whenever the context's launches change (ehd_set_tuning), so that
 // captured graphs holding them are rebuilt
 unsigned ctx_generation(const ::ehd_ctx *c);

@@ -1827,8 +1827,8 @@ cudaError_t prepare_poisson(const PoissonArgs &a) {
     cudaError_t e = allow_max_dynamic_smem(poisson_rows_fwd<R>);
     if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_rows_inv<R>);
     if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_cols<R>);
-    if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_zdst_rt<R>);
-    if (e == cudaSuccess) e = prepare_dft<R>(a.nx, a.ny);
+    if (e == cudaSuccess && a.ztb > 0) e = allow_max_dynamic_smem(poisson_zdst_rt<R>);
+    if (e == cudaSuccess && (a.tabx || a.taby || a.cpt)) e = prepare_dft<R>(a.nx, a.ny);
     if (e == cudaSuccess) e = prepare_fast<R>(a.nx);
     if (e == cudaSuccess) e = prepare_fast<R>(a.ny);
     if (e == cudaSuccess) e = prepare_fast<R>(2 * (a.nz - 1));
