@@ -43,6 +43,7 @@ namespace ehd {
 template <typename T, typename R, bool GENERAL, bool MACROS>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4)
 lbm_step_kernel(const StepArgs<T, R> a, const KConst<R> c, int local_pops, int e_arrays) {
+    step_enter();
     node_block<T, R, GENERAL, MACROS>(a, c, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x,
                                       gridDim.y, local_pops, e_arrays);
 }
@@ -216,6 +217,7 @@ __device__ __forceinline__ void rows_cta(const StepArgs<T, R> &a, const KConst<R
 template <typename T, typename R, bool MACROS, bool PART>
 __global__ void __launch_bounds__(256, sizeof(R) == 8 ? 1 : 2)
 lbm_rows_kernel(const StepArgs<T, R> a, const KConst<R> c) {
+    step_enter();
     rows_cta<T, R, MACROS, PART>(a, c);
 }
 
@@ -499,13 +501,13 @@ cudaError_t launch_lbm_step(const LbmArgs &la, const StepConst &c, int local_pop
         // (its shared-memory attribute was set by prepare_lbm_rows)
         const size_t sm = lbm_rows_smem(c.nx, sizeof(typename PopT<T>::F), sizeof(typename PopT<T>::G));
         const int tx = rows_block_x(c.nx);
-        rows_kernel<T, R>(macros, c.nx % 32 != 0)<<<c.ny + la.rows_grid, tx, sm, s>>>(a, k);
+        step_launch(rows_kernel<T, R>(macros, c.nx % 32 != 0), c.ny + la.rows_grid, tx, sm, s, a, k);
         return cudaGetLastError();
     }
     const int bx = la.node_bx > 0 ? la.node_bx : lbm_default_block_x(c.nx);
     dim3 block(bx, 128 / bx, 1);
     dim3 grid((c.nx + block.x - 1) / block.x, (c.ny + block.y - 1) / block.y, c.nz);
-#define EHD_LAUNCH(G, M) lbm_step_kernel<T, R, G, M><<<grid, block, 0, s>>>(a, k, local_pops, e_arrays)
+#define EHD_LAUNCH(G, M) step_launch(lbm_step_kernel<T, R, G, M>, grid, block, 0, s, a, k, local_pops, e_arrays)
     if (general) {
         if (macros) EHD_LAUNCH(true, true);
         else EHD_LAUNCH(true, false);
@@ -709,6 +711,7 @@ __global__ void __launch_bounds__(256)
 reduce_tables_kernel(const float2 *__restrict__ psum, double *__restrict__ m, int nblk0, int nblk,
                      long long nxy, const double *__restrict__ msrc, double *wdst,
                      const double *wread, R *__restrict__ ktab, int nz) {
+    step_enter();
     if ((int)blockIdx.x < nz) psum_reduce_block(psum, m, nblk0, nblk, nxy, blockIdx.x);
     else build_tables_block<R>(msrc, wdst, wread, ktab, nz);
 }
@@ -747,7 +750,7 @@ template <typename R>
 cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk0, int nblk,
                                  const double *msrc, double *wdst, const double *wread,
                                  void *ktab, const StepConst &c, cudaStream_t s) {
-    reduce_tables_kernel<R><<<c.nz + 1, 256, 0, s>>>(psum, m, nblk0, nblk, c.nxy, msrc, wdst, wread,
+    step_launch(reduce_tables_kernel<R>, c.nz + 1, 256, 0, s, psum, m, nblk0, nblk, c.nxy, msrc, wdst, wread,
                                                      (R *)ktab, c.nz);
     return cudaGetLastError();
 }

@@ -107,6 +107,7 @@ __device__ __forceinline__ void plane0_block(const StepArgs<T, float> &a, const 
 template <typename T, bool MACROS>
 __global__ void __launch_bounds__(kPairThreads, 4)
 lbm_plane0_kernel(const StepArgs<T, float> a, const KConst<float> c) {
+    step_enter();
     plane0_block<T, MACROS>(a, c, blockIdx.x);
 }
 
@@ -115,6 +116,7 @@ lbm_plane0_kernel(const StepArgs<T, float> a, const KConst<float> c) {
 template <typename T, bool MACROS, typename Args>
 __global__ void __launch_bounds__(kPairThreads, 3)
 lbm_pair_kernel(const Args a, const KConst<float> c) {
+    step_enter();
     constexpr bool kPlane0 = std::is_same<Args, StepArgs<T, float>>::value;
     const int NX = c.nx, NY = c.ny, NZ = c.nz, hx = NX / 2;
     const int pairs = hx * NY;
@@ -349,8 +351,8 @@ static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macro
     const int pairs = c.nx / 2 * c.ny, nb = (pairs + kPairThreads - 1) / kPairThreads;
     if (nb * (long long)(c.nz - 1) <= kMergeBlocks) {
         const dim3 grid(nb, c.nz + 1);
-        if (macros) lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(a, k);
-        else lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(a, k);
+        if (macros) step_launch(lbm_pair_kernel<T, true, StepArgs<T, float>>, grid, kPairThreads, 0, s, a, k);
+        else step_launch(lbm_pair_kernel<T, false, StepArgs<T, float>>, grid, kPairThreads, 0, s, a, k);
         return cudaGetLastError();
     }
     PairArgs<T> p;
@@ -366,11 +368,11 @@ static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macro
     p.psum = a.psum + 2 * lbm_pair_slots(c.nx, c.ny);
     const dim3 grid(nb, c.nz - 1);
     if (macros) {
-        lbm_plane0_kernel<T, true><<<2 * nb, kPairThreads, 0, s>>>(a, k);
-        lbm_pair_kernel<T, true><<<grid, kPairThreads, 0, s>>>(p, k);
+        step_launch(lbm_plane0_kernel<T, true>, 2 * nb, kPairThreads, 0, s, a, k);
+        step_launch(lbm_pair_kernel<T, true, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
     } else {
-        lbm_plane0_kernel<T, false><<<2 * nb, kPairThreads, 0, s>>>(a, k);
-        lbm_pair_kernel<T, false><<<grid, kPairThreads, 0, s>>>(p, k);
+        step_launch(lbm_plane0_kernel<T, false>, 2 * nb, kPairThreads, 0, s, a, k);
+        step_launch(lbm_pair_kernel<T, false, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
     }
     return cudaGetLastError();
 }

@@ -216,6 +216,7 @@ poisson_rows_fwd(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec
                  const double *__restrict__ qmean, FftPlan pl, int nx, int ny, int nxh, int pitch,
                  int rows, double eps,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         q = (const R *)gp.q;
@@ -286,6 +287,7 @@ poisson_cols(typename Cplx<R>::T *__restrict__ spec, const typename Cplx<R>::T *
              FftPlan pl, int ny, int nxh, int pitch, int cols, R sign,
              const double *__restrict__ rowsum, double *__restrict__ planesum,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (typename Cplx<R>::T *)gp.spec;
@@ -327,6 +329,7 @@ poisson_rows_inv(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ p
                  const typename Cplx<R>::T *__restrict__ tw, FftPlan pl, int nx, int ny,
                  int nxh, int pitch, int rows,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (const typename Cplx<R>::T *)gp.spec;
@@ -399,6 +402,7 @@ poisson_rows_fwd_fast(const R *__restrict__ q, typename Cplx<R>::T *__restrict__
                       double *__restrict__ rowsum, const typename Cplx<R>::T *__restrict__ tw,
                       const double *__restrict__ qmean, int ny, int nxh, int pitch, double eps,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         q = (const R *)gp.q;
@@ -472,6 +476,7 @@ poisson_cols_fast(typename Cplx<R>::T *__restrict__ spec,
                   const typename Cplx<R>::T *__restrict__ tw, int nxh, int pitch,
                   const double *__restrict__ rowsum, double *__restrict__ planesum,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (typename Cplx<R>::T *)gp.spec;
@@ -521,6 +526,7 @@ __global__ void __launch_bounds__(256)
 poisson_rows_inv_fast(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phip,
                       const typename Cplx<R>::T *__restrict__ tw, int ny, int nxh, int pitch,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (const typename Cplx<R>::T *)gp.spec;
@@ -603,6 +609,7 @@ poisson_zsolve(typename Cplx<R>::T *__restrict__ spec, const double *__restrict_
                double *__restrict__ ez00, int nx, int ny, int nz, int nxh, int pitch,
                double dz, double eps, double voltage,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (typename Cplx<R>::T *)gp.spec;
@@ -725,6 +732,7 @@ poisson_zdst(typename Cplx<R>::T *__restrict__ spec, const typename Cplx<R>::T *
              double *__restrict__ ez00, int nx, int ny, int nxh, int pitch, double dz,
              double eps, double voltage, double kx0, double ky0,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (typename Cplx<R>::T *)gp.spec;
@@ -865,6 +873,7 @@ poisson_zdst_rt(typename Cplx<R>::T *__restrict__ spec, const typename Cplx<R>::
                 double *__restrict__ ez00, int nx, int ny, int nxh, int pitch, int tb, double dz,
                 double eps, double voltage, double kx0, double ky0,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spec = (typename Cplx<R>::T *)gp.spec;
@@ -1053,6 +1062,7 @@ poisson_rows_fwd_split(const R *__restrict__ q, typename Cplx<R>::T *__restrict_
                        const typename Cplx<R>::T *__restrict__ twy,
                        const double *__restrict__ qmean, int nzi, int nxh, double eps,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         q = (const R *)gp.q;
@@ -1223,6 +1233,7 @@ poisson_slab(typename Cplx<R>::T *__restrict__ spl, const typename Cplx<R>::T *_
              double *__restrict__ planesum, const double *__restrict__ qmean,
              double *__restrict__ phi00, double *__restrict__ ez00, int nx, int nxh, double dz,
              double eps, double voltage, const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spl = (typename Cplx<R>::T *)gp.spec;
@@ -1440,6 +1451,7 @@ poisson_rows_inv_split(const typename Cplx<R>::T *__restrict__ spl, R *__restric
                        const typename Cplx<R>::T *__restrict__ tw,
                        const typename Cplx<R>::T *__restrict__ twy, int nzi, int nxh,
     const PoissonPtrs *__restrict__ grp) {
+    step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
         spl = (const typename Cplx<R>::T *)gp.spec;
@@ -1548,7 +1560,7 @@ static cudaError_t rows_fwd_fast(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_rows_fwd_fast<R, N>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * TB - 1) / (2 * TB), a.nz - 2, a.ngrp);
-    poisson_rows_fwd_fast<R, N><<<grid, 256, sm, s>>>((const R *)a.q, (R2 *)a.spec, a.rowsum,
+    step_launch(poisson_rows_fwd_fast<R, N>, grid, 256, sm, s, (const R *)a.q, (R2 *)a.spec, a.rowsum,
                                                        (const R2 *)a.twx, a.qmean,
                                                        a.ny, a.nxh, a.pitch, a.eps, a.grp);
     return cudaGetLastError();
@@ -1561,7 +1573,7 @@ static cudaError_t rows_inv_fast(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_rows_inv_fast<R, N>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * TB - 1) / (2 * TB), a.nz - 2, a.ngrp);
-    poisson_rows_inv_fast<R, N><<<grid, 256, sm, s>>>((const R2 *)a.spec, (R *)a.phip,
+    step_launch(poisson_rows_inv_fast<R, N>, grid, 256, sm, s, (const R2 *)a.spec, (R *)a.phip,
                                                        (const R2 *)a.twx, a.ny, a.nxh, a.pitch, a.grp);
     return cudaGetLastError();
 }
@@ -1573,7 +1585,7 @@ static cudaError_t cols_fast(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_cols_fast<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nxh + TB - 1) / TB, a.nz - 2, a.ngrp);
-    poisson_cols_fast<R, N, S><<<grid, 256, sm, s>>>((R2 *)a.spec, (const R2 *)a.twy, a.nxh,
+    step_launch(poisson_cols_fast<R, N, S>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy, a.nxh,
                                                       a.pitch, a.rowsum, a.planesum, a.grp);
     return cudaGetLastError();
 }
@@ -1597,7 +1609,7 @@ static cudaError_t rows_fwd(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_rows_fwd<R>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * rows - 1) / (2 * rows), a.nz - 2, a.ngrp);
-    poisson_rows_fwd<R><<<grid, 256, sm, s>>>((const R *)a.q, (R2 *)a.spec, a.rowsum,
+    step_launch(poisson_rows_fwd<R>, grid, 256, sm, s, (const R *)a.q, (R2 *)a.spec, a.rowsum,
                                                (const R2 *)a.twx, a.qmean, a.px,
                                                a.nx, a.ny, a.nxh, a.pitch, rows, a.eps, a.grp);
     return cudaGetLastError();
@@ -1621,7 +1633,7 @@ static cudaError_t rows_inv(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_rows_inv<R>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * rows - 1) / (2 * rows), a.nz - 2, a.ngrp);
-    poisson_rows_inv<R><<<grid, 256, sm, s>>>((const R2 *)a.spec, (R *)a.phip,
+    step_launch(poisson_rows_inv<R>, grid, 256, sm, s, (const R2 *)a.spec, (R *)a.phip,
                                                (const R2 *)a.twx, a.px, a.nx, a.ny, a.nxh,
                                                a.pitch, rows, a.grp);
     return cudaGetLastError();
@@ -1645,7 +1657,7 @@ static cudaError_t cols(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_cols<R>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nxh + cc - 1) / cc, a.nz - 2, a.ngrp);
-    poisson_cols<R><<<grid, 256, sm, s>>>((R2 *)a.spec, (const R2 *)a.twy, a.py, a.ny, a.nxh,
+    step_launch(poisson_cols<R>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy, a.py, a.ny, a.nxh,
                                            a.pitch, cc, (R)S, S < 0 ? a.rowsum : nullptr,
                                            S < 0 ? a.planesum : nullptr, a.grp);
     return cudaGetLastError();
@@ -1660,7 +1672,7 @@ static cudaError_t zdst(const PoissonArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int modes = a.nxh * a.ny;
     const R2 *tw = (const R2 *)a.twz;
-    poisson_zdst<R, L><<<dim3((modes + TB - 1) / TB, 1, a.ngrp), 256, sm, s>>>(
+    step_launch(poisson_zdst<R, L>, dim3((modes + TB - 1) / TB, 1, a.ngrp), 256, sm, s, 
         (R2 *)a.spec, tw, (const R *)(tw + L), a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny,
         a.nxh, a.pitch, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx, 2.0 * M_PI / a.ly, a.grp);
     return cudaGetLastError();
@@ -1681,7 +1693,7 @@ static cudaError_t split_rows_fwd(const PoissonArgs &a, cudaStream_t s) {
     const size_t sm = sizeof(R2) * ((size_t)N + (size_t)TB * tstride<N>());
     cudaError_t e = set_smem(poisson_rows_fwd_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
-    poisson_rows_fwd_split<R, N, S><<<dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s>>>(
+    step_launch(poisson_rows_fwd_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s, 
         (const R *)a.q, (R2 *)a.spec, a.rowsum, (const R2 *)a.twx, (const R2 *)a.twy, a.qmean,
         a.nz - 2, a.nxh, a.eps, a.grp);
     return cudaGetLastError();
@@ -1693,7 +1705,7 @@ static cudaError_t split_rows_inv(const PoissonArgs &a, cudaStream_t s) {
     constexpr size_t sm = rows_inv_split_smem<R, N, S>();
     cudaError_t e = set_smem(poisson_rows_inv_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
-    poisson_rows_inv_split<R, N, S><<<dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s>>>(
+    step_launch(poisson_rows_inv_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s, 
         (const R2 *)a.spec, (R *)a.phip, (const R2 *)a.twx, (const R2 *)a.twy, a.nz - 2, a.nxh, a.grp);
     return cudaGetLastError();
 }
@@ -1704,7 +1716,7 @@ static cudaError_t split_slab(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_slab<R, L, S>, sm, s);
     if (e != cudaSuccess) return e;
     // one block more than kx columns: block x = 0 solves the mean mode
-    poisson_slab<R, L, S><<<dim3(a.nxh + 1, S, a.ngrp), 256, sm, s>>>(
+    step_launch(poisson_slab<R, L, S>, dim3(a.nxh + 1, S, a.ngrp), 256, sm, s, 
         (R2 *)a.spec, (const R2 *)a.twy, (const R *)a.cps, a.rowsum, a.planesum, a.qmean,
         a.phi00, a.ez00, a.nx, a.nxh, a.dz, a.eps, a.voltage, a.grp);
     return cudaGetLastError();
@@ -1875,14 +1887,14 @@ static cudaError_t zsolve(const PoissonArgs &a0, cudaStream_t s) {
         cudaError_t e = set_smem(poisson_zdst_rt<R>, sm, s);
         if (e != cudaSuccess) return e;
         const R2 *tw = (const R2 *)a.twz;
-        poisson_zdst_rt<R><<<dim3((modes + a.ztb - 1) / a.ztb, 1, a.ngrp), 256, sm, s>>>(
+        step_launch(poisson_zdst_rt<R>, dim3((modes + a.ztb - 1) / a.ztb, 1, a.ngrp), 256, sm, s, 
             (R2 *)a.spec, tw, (const R *)(tw + L), a.pz, a.planesum, a.qmean, a.phi00, a.ez00,
             a.nx, a.ny, a.nxh, a.pitch, a.ztb, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx,
             2.0 * M_PI / a.ly, a.grp);
         return cudaGetLastError();
     }
     if (!a.thomas && zmeet_modes(a.nz, sizeof(R)) > 0) return launch_zmeet<R>(a, s);
-    poisson_zsolve<R><<<dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s>>>(
+    step_launch(poisson_zsolve<R>, dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s, 
         (R2 *)a.spec, a.cpt, a.dpw, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz,
         a.nxh, a.pitch, a.dz, a.eps, a.voltage, a.grp);
     return cudaGetLastError();
