@@ -8,9 +8,10 @@
 // the whole state and runs any number of steps in one launch, so that a step
 // costs its own chain of dependent operations.  Measured, FP64: a column of NZ = 33
 // run 16,000 steps through ehd_hydrostatic_profile, its context's creation
-// included, 388 -> 30 ms (24.3 -> 1.9 us a step); 12 columns of NZ = 25 as one
-// batch, 12,000 steps, 609 -> 44 ms (one block per column, side by side, where
-// the batch's graph had held 84 launches a step).
+// included, 388 -> 26 ms (24.3 -> 1.6 us a step; 30 ms with the moments as
+// chains of additions and divisions by constants in the loop); 12 columns of
+// NZ = 25 as one batch, 12,000 steps, 609 -> 38 ms (one block per column, side
+// by side, where the batch's graph had held 84 launches a step).
 //
 // Thread z of the first half of the block holds node z's flow populations f
 // in registers, thread z of the second half its charge populations g (the two
@@ -71,6 +72,23 @@ __device__ __forceinline__ R dot_dir(int d, R a, R b, R c) {
     return s;
 }
 
+// Sum of the products sign(d) v_d, sign in {-1, 0, 1}, as a tree: a chain of
+// 27 FP64 additions would be the longest part of a step.
+template <typename R, typename S>
+__device__ __forceinline__ R tree_sum(const R (&v)[Q], S sign) {
+    R t[Q];
+    int n = 0;
+#pragma unroll
+    for (int d = 0; d < Q; ++d)
+        if (sign(d) != 0) t[n++] = sign(d) > 0 ? v[d] : -v[d];
+#pragma unroll
+    for (int w = 1; w < Q; w *= 2)
+#pragma unroll
+        for (int i = 0; i + w < Q; i += 2 * w)
+            if (i + w < n) t[i] += t[i + w];
+    return t[0];
+}
+
 }  // namespace
 
 // dynamic shared memory, for nz nodes:
@@ -103,7 +121,8 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
     const int lane = threadIdx.x & 31, gw = z >> 5;  // warp of this half
     const int zc = act ? z : nz - 1;
     const int zm = zc == 0 ? nz - 1 : zc - 1, zp = zc == nz - 1 ? 0 : zc + 1;
-    const double dz = a.dz, dz2 = a.dz * a.dz;
+    // (no division in the loop but 1 / rho)
+    const double kD = -(a.dz * a.dz) / a.eps, kN = 1.0 / (double)(n + 1), kE = 0.5 / a.dz;
 
     int p = a.parity;
     for (int i = threadIdx.x; i < 2 * nz; i += blockDim.x) {
@@ -148,23 +167,18 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
             dr[0] = (R)(rd[2 * zp] - rw);
             dr[1] = (R)(rd[2 * zc] - rw);
             dr[2] = (R)(rd[2 * zm] - rw);
-            R mx = 0, my = 0, mz = 0;
-            dev = 0;
 #pragma unroll
             for (int d = 0; d < Q; ++d) {
                 const int e = ez_of(d);
                 const R v = e == 0 ? s[d] : xf[mov_of(d) * nz + (e > 0 ? zm : zp)];
                 s[d] = v + c.w[cls_of(d)] * dr[e + 1];
-                dev += s[d];
-                if (ex_of(d)) mx += ex_of(d) > 0 ? s[d] : -s[d];
-                if (ey_of(d)) my += ey_of(d) > 0 ? s[d] : -s[d];
-                if (ez_of(d)) mz += ez_of(d) > 0 ? s[d] : -s[d];
             }
+            dev = tree_sum(s, [](int) { return 1; });
             rho = rref + dev;
             if (act) {
-                mom[z] = mx;
-                mom[nz + z] = my;
-                mom[2 * nz + z] = mz;
+                mom[z] = tree_sum(s, [](int d) { return ex_of(d); });
+                mom[nz + z] = tree_sum(s, [](int d) { return ey_of(d); });
+                mom[2 * nz + z] = tree_sum(s, [](int d) { return ez_of(d); });
                 mom[3 * nz + z] = rho;
             }
         } else {
@@ -177,20 +191,16 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
 #pragma unroll
                 for (int d = 0; d < Q; ++d) s[d] = top[d];
             }
-            dev = 0;
             if (z == 0) {
                 // the injector: g_d = -g_opp(d) + 2 q0 w_d of its own values
                 // (LBM.cu:1320-1348), on deviations
                 const R inj = (R)2 * (c.q0 - qref) - dq[1];
                 s[0] += c.w[0] * dq[1];
-                dev = s[0];
 #pragma unroll
                 for (int d = 1; d < Q; d += 2) {
                     const R t = s[d];
                     s[d] = -s[d + 1] + inj * c.w[cls_of(d)];
                     s[d + 1] = -t + inj * c.w[cls_of(d)];
-                    dev += s[d];
-                    dev += s[d + 1];
                 }
             } else {
 #pragma unroll
@@ -198,13 +208,13 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                     const int e = ez_of(d);
                     const R v = e == 0 ? s[d] : xg[mov_of(d) * nz + (e > 0 ? zm : zp)];
                     s[d] = v + c.w[cls_of(d)] * dq[e + 1];
-                    dev += s[d];
                 }
             }
+            dev = tree_sum(s, [](int) { return 1; });
             charge = qref + dev;
             if (act) chg[z] = charge;
             // the warp's prefix sum of D and sum of (n + 1 - z) D
-            D = act && z >= 1 && z <= n ? -(double)charge / a.eps * dz2 : 0.0;
+            D = act && z >= 1 && z <= n ? (double)charge * kD : 0.0;
             P = D;
             double W = (double)(n + 1 - z) * D;
 #pragma unroll
@@ -299,8 +309,8 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                     W += wsum[2 * w + 1];
                 }
                 P += off;
-                s0 = (a.voltage + W) / (double)(n + 1);
-                const double e = 0.5 * (2.0 * s0 - 2.0 * P + D) / dz;
+                s0 = (a.voltage + W) * kN;
+                const double e = (2.0 * s0 - 2.0 * P + D) * kE;
                 if (z >= 1 && z <= n) ez_next[z] = e;
                 if (z == 1) ez_next[0] = e;
                 if (z == n) ez_next[nz - 1] = e;
@@ -381,7 +391,7 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
         // phi_z = V - (s_0 + .. + s_{z-1})
         double ph = a.voltage, edge = s0;
         for (int i = 0; i < z; ++i) {
-            if (i >= 1) edge += (double)chg[i] / a.eps * dz2;
+            if (i >= 1) edge -= (double)chg[i] * kD;
             ph -= edge;
         }
         a.phi00[z] = z == nz - 1 ? 0.0 : ph;
