@@ -12,6 +12,12 @@
 // allocating.  It calls no cudaMalloc, cudaFree or other allocating routine,
 // on the device or on the host.
 //
+// A call is seven launches: the tables in one, the five of the solve, phi and E
+// in one, each waiting on the one before as the step's do.  With 13 launches
+// (tables, three memsets, an E kernel of one warp a block, phi in place) a call
+// at 96 x 96 x 65 took 64 us, so 38 (109 before that with the one-thread-per-mode
+// FP64 sweep).
+//
 // The array costs EHD_NOALLOC_SCRATCH_BYTES of device memory on each GPU the
 // entry point is used on, until the process exits.  Under CUDA's lazy module
 // loading (the default) the driver commits it when the first call on a device
@@ -82,61 +88,63 @@ FftPlan plan_of(int n) {
     return p;
 }
 
-// exp(-2 pi i k / n), FP64
-__global__ void twiddle_kernel(double2 *tw, int n) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        double s, c;
-        sincospi(-2.0 * (double)k / (double)n, &s, &c);
-        tw[k] = make_double2(c, s);
-    }
-}
-
-// Thomas pivots per mode, the same table as the context's (api.cu):
-// beta = 2 + (kx^2 + ky^2) dz^2, cp_0 = -1/beta, cp_i = 1/(-beta - cp_{i-1}).
-__global__ void pivot_kernel(double *cpt, int nx, int ny, int nz, double lx, double ly,
-                             double dz) {
+// Everything the solve reads before writing, in one launch: the twiddles
+// exp(-2 pi i k / n) of both axes, the zero reference charge, and the Thomas
+// pivots per mode, the same table as the context's (api.cu):
+// beta = 2 + (kx^2 + ky^2) dz^2, cp_0 = -1/beta, cp_i = 1/(-beta - cp_{i-1}),
+// the first `rows` of them (one thread a mode, the thread's number also that
+// of a twiddle or reference).
+__global__ void setup_kernel(double2 *twx, double2 *twy, double *qmean, double *cpt, int nx, int ny,
+                             int nz, int rows, double lx, double ly, double dz) {
     const int nxh = nx / 2 + 1;
     const int modes = nxh * ny;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    const int stride = gridDim.x * blockDim.x;
+    for (int k = m; k < nx + ny; k += stride) {
+        const bool xa = k < nx;
+        const int i = xa ? k : k - nx;
+        double s, c;
+        sincospi(-2.0 * (double)i / (double)(xa ? nx : ny), &s, &c);
+        (xa ? twx : twy)[i] = make_double2(c, s);
+    }
+    for (int k = m; k < 2 * nz; k += stride) qmean[k] = 0.0;
     if (m >= modes) return;
     const int j = m / nxh, i = m - j * nxh;
     const double kx = (double)i * 2.0 * M_PI / lx;
     const double ky = (j <= ny / 2 ? (double)j : (double)j - ny) * 2.0 * M_PI / ly;
     const double beta = 2.0 + (kx * kx + ky * ky) * dz * dz;
     double prev = 0.0;
-    for (int z = 0; z < nz - 2; ++z) {
+    for (int z = 0; z < rows; ++z) {
         prev = 1.0 / (-beta - prev);
         cpt[(size_t)z * modes + m] = prev;
     }
 }
 
-// E = -grad(phi) from phi' (in phi) and phi00, central differences with the
-// electrode copy of Ez (gpu_efield, gpu_bc, poisson.cu:44-73).
-__global__ void efield_kernel(const double *__restrict__ phip, const double *__restrict__ phi00,
-                              double *__restrict__ ex, double *__restrict__ ey,
-                              double *__restrict__ ez, int nx, int ny, int nz, double dx,
-                              double dy, double dz) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y, z = blockIdx.z;
-    if (x >= nx) return;
-    auto idx = [&](int xx, int yy, int zz) {
-        return (size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz);
+// phi = phi00(z) + phi' (phi00 carries V and 0 on the electrodes, phi' is zero
+// there) and E = -grad(phi), central differences with the electrode copy of
+// Ez (gpu_efield, gpu_bc, poisson.cu:44-73), from phi' of the planes 1..NZ-2
+// in scratch (phip points a plane before them).
+__global__ void fields_kernel(const double *__restrict__ phip, const double *__restrict__ phi00,
+                              double *__restrict__ phi, double *__restrict__ ex,
+                              double *__restrict__ ey, double *__restrict__ ez, int nx, int ny,
+                              int nz, double inv2dx, double inv2dy, double inv2dz) {
+    step_enter();
+    // runs over a plane: rows alone would be short blocks on narrow grids
+    const int xy = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y;
+    if (xy >= nx * ny) return;
+    const int y = xy / nx, x = xy - y * nx;
+    auto p = [&](int xx, int yy, int zz) {
+        return zz == 0 || zz == nz - 1 ? 0.0
+                                       : __ldg(phip + (size_t)xx + (size_t)nx * ((size_t)yy + (size_t)ny * zz));
     };
-    auto phi = [&](int xx, int yy, int zz) { return phi00[zz] + phip[idx(xx, yy, zz)]; };
-    const int xm = (nx + x - 1) % nx, xp = (x + 1) % nx;
-    const int ym = (ny + y - 1) % ny, yp = (y + 1) % ny;
+    const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
+    const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
     const int zc = z < 1 ? 1 : (z > nz - 2 ? nz - 2 : z);
-    const size_t i = idx(x, y, z);
-    ex[i] = 0.5 * (phi(xm, y, z) - phi(xp, y, z)) / dx;
-    ey[i] = 0.5 * (phi(x, ym, z) - phi(x, yp, z)) / dy;
-    ez[i] = 0.5 * (phi(x, y, zc - 1) - phi(x, y, zc + 1)) / dz;
-}
-
-// phi = phi00(z) + phi' in place (phi00 carries V and 0 on the electrodes).
-__global__ void phi_kernel(double *__restrict__ phi, const double *__restrict__ phi00,
-                           long long nxy, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) phi[i] = phi00[i / nxy] + phi[i];
+    const size_t i = (size_t)x + (size_t)nx * ((size_t)y + (size_t)ny * z);
+    phi[i] = phi00[z] + p(x, y, z);
+    ex[i] = (p(xm, y, z) - p(xp, y, z)) * inv2dx;
+    ey[i] = (p(x, ym, z) - p(x, yp, z)) * inv2dy;
+    ez[i] = ((phi00[zc - 1] + p(x, y, zc - 1)) - (phi00[zc + 1] + p(x, y, zc + 1))) * inv2dz;
 }
 
 }  // namespace
@@ -231,33 +239,26 @@ extern "C" int ehd_poisson_noalloc(const ehd_params *p, const double *q, double 
     a.twy = twy;
     a.q = q;
     a.qmean = qmean;
-    a.phip = phi;  // phi' is built in the caller's phi array, then completed
+    // phi' of the interior planes into the sweep's scratch, which is free by then
+    // (16 bytes a mode and plane; the solve writes plane z at phip + z NX NY)
+    double *phip = (double *)a.dpw - (size_t)nx * ny;
+    a.phip = phip;
     a.eps = p->eps;
     a.voltage = p->voltage;
     a.dz = p->dz;
     a.lx = p->lx;
     a.ly = p->ly;
 
-    const size_t nxy = (size_t)nx * ny;
-    // every region the solve reads before writing is set here: the tables,
-    // the zero reference charge, and phi' = 0 on both electrodes
-    twiddle_kernel<<<(nx + 255) / 256, 256, 0, s>>>(twx, nx);
-    twiddle_kernel<<<(ny + 255) / 256, 256, 0, s>>>(twy, ny);
-    pivot_kernel<<<(unsigned)((modes + 127) / 128), 128, 0, s>>>(cpt, nx, ny, nz, p->lx, p->ly,
-                                                                  p->dz);
+    // the two-sided z solve reads the pivots of half the planes
+    const int piv = zmeet_modes(nz, sizeof(double)) > 0 ? (nz - 2) / 2 : nz - 2;
+    setup_kernel<<<(unsigned)((modes + 127) / 128), 128, 0, s>>>(twx, twy, qmean, cpt, nx, ny, nz, piv,
+                                                                  p->lx, p->ly, p->dz);
     if (cudaGetLastError() != cudaSuccess)
-        return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: table kernels failed to launch");
-    if (cudaMemsetAsync(qmean, 0, sizeof(double) * 2 * nz, s) != cudaSuccess ||
-        cudaMemsetAsync(phi, 0, sizeof(double) * nxy, s) != cudaSuccess ||
-        cudaMemsetAsync(phi + (size_t)(nz - 1) * nxy, 0, sizeof(double) * nxy, s) != cudaSuccess)
-        return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: cudaMemsetAsync failed");
+        return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: the table kernel failed to launch");
     if (launch_poisson<double>(a, s) != cudaSuccess)
         return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: Poisson kernels failed to launch");
-    dim3 blk(nx >= 128 ? 128 : 32), grd((nx + blk.x - 1) / blk.x, ny, nz);
-    efield_kernel<<<grd, blk, 0, s>>>(phi, a.phi00, ex, ey, ez, nx, ny, nz, p->dx, p->dy, p->dz);
-    const long long n = (long long)nxy * nz;
-    phi_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(phi, a.phi00, (long long)nxy, n);
-    if (cudaGetLastError() != cudaSuccess)
-        return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: field kernels failed to launch");
+    if (step_launch(fields_kernel, dim3((nx * ny + 255) / 256, nz), 256, 0, s, phip, a.phi00, phi, ex, ey, ez, nx, ny, nz,
+                    0.5 / p->dx, 0.5 / p->dy, 0.5 / p->dz) != cudaSuccess)
+        return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: the field kernel failed to launch");
     return EHD_OK;
 }
