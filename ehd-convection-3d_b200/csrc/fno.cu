@@ -43,6 +43,7 @@ struct Off {  // offsets of one layer's parameters in the FP32 vector
 
 __global__ void cast_bf16_kernel(const float *__restrict__ src, __nv_bfloat16 *__restrict__ dst,
                                  size_t n) {
+    step_enter();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x)
         dst[i] = __float2bfloat16_rn(src[i]);
@@ -65,6 +66,7 @@ __host__ __device__ inline size_t mix_warp_floats(int W) {
 __global__ void mix_kernel(const float *__restrict__ re, const float *__restrict__ im,
                            const float *__restrict__ in, float *__restrict__ out, int modes, int W,
                            int B, int adj) {
+    step_enter();
     extern __shared__ float mix_smem[];
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int WP = W + 1;
@@ -135,6 +137,7 @@ template <int WT>
 __global__ void mix_kernel_w(const float *__restrict__ re, const float *__restrict__ im,
                              const float *__restrict__ in, float *__restrict__ out, int modes,
                              int B, int adj) {
+    step_enter();
     constexpr int W = WT, WP = W + 1, V = (W * W + 31) / 32, XV = (8 * W + 31) / 32;
     extern __shared__ float mix_smem[];
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -212,6 +215,7 @@ __global__ void mix_kernel_w(const float *__restrict__ re, const float *__restri
 __global__ void mix_wgrad_kernel(const float *__restrict__ dout, const float *__restrict__ x,
                                  float *__restrict__ gre, float *__restrict__ gim, int modes,
                                  int W, int B) {
+    step_enter();
     extern __shared__ float mix_smem[];
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float *D = mix_smem + (size_t)warp * 16 * W;  // [4][re, im][W]
@@ -261,6 +265,7 @@ __global__ void mix_wgrad_kernel(const float *__restrict__ dout, const float *__
 
 // d *= gelu'(z)
 __global__ void gelu_back_kernel(float *__restrict__ d, const float *__restrict__ z, size_t n) {
+    step_enter();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x)
         d[i] *= gelu_grad(z[i]);
@@ -272,6 +277,7 @@ __device__ __forceinline__ float4 gelu_back4(float4 a, float4 b) {
 // the same on 16-byte vectors (both arrays 16-byte aligned, n4 = n / 4), two
 // vectors a thread in flight per iteration; elementwise the same arithmetic
 __global__ void gelu_back4_kernel(float4 *__restrict__ d, const float4 *__restrict__ z, size_t n4) {
+    step_enter();
     const size_t st = (size_t)gridDim.x * blockDim.x;
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     for (; i + st < n4; i += 2 * st) {
@@ -286,6 +292,7 @@ __global__ void gelu_back4_kernel(float4 *__restrict__ d, const float4 *__restri
 // before one atomic addition per block (256 threads)
 __global__ void mse_kernel(const float *__restrict__ u, const float *__restrict__ t,
                            float *__restrict__ du, size_t n, double *sum) {
+    step_enter();
     __shared__ double ws[8];
     double s = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
@@ -314,6 +321,7 @@ __device__ __forceinline__ void adam_one(float &p, float g, float &m, float &v, 
 __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g,
                             float *__restrict__ m, float *__restrict__ v, size_t n, float lr,
                             float b1, float b2, float eps, float c1, float c2) {
+    step_enter();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x) {
         float pi = p[i], mi = m[i], vi = v[i];
@@ -328,6 +336,7 @@ __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g,
 __global__ void adam4_kernel(float *__restrict__ p, const float *__restrict__ g,
                              float *__restrict__ m, float *__restrict__ v, size_t n, float lr,
                              float b1, float b2, float eps, float c1, float c2) {
+    step_enter();
     const size_t n4 = n / 4;
     float4 *p4 = reinterpret_cast<float4 *>(p), *m4 = reinterpret_cast<float4 *>(m),
            *v4 = reinterpret_cast<float4 *>(v);
@@ -361,10 +370,10 @@ bool aligned16(const void *a) { return ((uintptr_t)a & 15) == 0; }
 // d *= gelu'(z) over n elements, on vectors where the layout allows
 void gelu_back(float *d, const float *z, size_t n, cudaStream_t s) {
     if (n % 4 == 0 && aligned16(d) && aligned16(z))
-        gelu_back4_kernel<<<grid_for(n / 8), 256, 0, s>>>(reinterpret_cast<float4 *>(d),
+        step_launch(gelu_back4_kernel, grid_for(n / 8), 256, 0, s, reinterpret_cast<float4 *>(d),
                                                          reinterpret_cast<const float4 *>(z), n / 4);
     else
-        gelu_back_kernel<<<grid_for(n), 256, 0, s>>>(d, z, n);
+        step_launch(gelu_back_kernel, grid_for(n), 256, 0, s, d, z, n);
 }
 
 }  // namespace
@@ -495,7 +504,7 @@ cudaError_t refresh(ehd_fno *f) {
     for (int l = 0; l <= f->L; ++l) {
         const size_t to = l < f->L ? f->lo[l].Rre : f->nparam;
         if (to > from)
-            cast_bf16_kernel<<<grid_for(to - from), 256, 0, f->stream>>>(f->param + from,
+            step_launch(cast_bf16_kernel, grid_for(to - from), 256, 0, f->stream, f->param + from,
                                                                          f->pbf + from, to - from);
         if (l < f->L) from = f->lo[l].Rim + spec;
     }
@@ -767,11 +776,11 @@ cudaError_t mix(const ehd_fno *f, int l, const float *in, float *out, int B, boo
     const float *re = f->param + f->lo[l].Rre, *im = f->param + f->lo[l].Rim;
     const int a = adj ? 1 : 0;
     if (B <= 4 && (f->W == 8 || f->W == 16 || f->W == 32)) {
-        if (f->W == 8) mix_kernel_w<8><<<blocks, 32 * nw, sm, f->stream>>>(re, im, in, out, f->modes, B, a);
-        else if (f->W == 16) mix_kernel_w<16><<<blocks, 32 * nw, sm, f->stream>>>(re, im, in, out, f->modes, B, a);
-        else mix_kernel_w<32><<<blocks, 32 * nw, sm, f->stream>>>(re, im, in, out, f->modes, B, a);
+        if (f->W == 8) step_launch(mix_kernel_w<8>, blocks, 32 * nw, sm, f->stream, re, im, in, out, f->modes, B, a);
+        else if (f->W == 16) step_launch(mix_kernel_w<16>, blocks, 32 * nw, sm, f->stream, re, im, in, out, f->modes, B, a);
+        else step_launch(mix_kernel_w<32>, blocks, 32 * nw, sm, f->stream, re, im, in, out, f->modes, B, a);
     } else {
-        mix_kernel<<<blocks, 32 * nw, sm, f->stream>>>(re, im, in, out, f->modes, f->W, B, a);
+        step_launch(mix_kernel, blocks, 32 * nw, sm, f->stream, re, im, in, out, f->modes, f->W, B, a);
     }
     return cudaGetLastError();
 }
@@ -779,7 +788,7 @@ cudaError_t mix(const ehd_fno *f, int l, const float *in, float *out, int B, boo
 cudaError_t mix_wgrad(const ehd_fno *f, int l, const float *dout, const float *x, float *g, int B) {
     const int nw = mix_warps(f->W, (size_t)16 * f->W);
     const unsigned blocks = (unsigned)std::min<size_t>((f->modes + nw - 1) / nw, 148 * 16);
-    mix_wgrad_kernel<<<blocks, 32 * nw, (size_t)nw * 16 * f->W * sizeof(float), f->stream>>>(
+    step_launch(mix_wgrad_kernel, blocks, 32 * nw, (size_t)nw * 16 * f->W * sizeof(float), f->stream, 
         dout, x, g + f->lo[l].Rre, g + f->lo[l].Rim, f->modes, f->W, B);
     return cudaGetLastError();
 }
@@ -1021,7 +1030,7 @@ int ehd_fno_backward(ehd_fno *f, int B, const float *a, const float *target, dou
     const __nv_bfloat16 *pb = f->pbf;
     FNO_CK(cudaMemsetAsync(g, 0, f->nparam * sizeof(float), s));
     FNO_CK(cudaMemsetAsync(f->lsum, 0, sizeof(double), s));
-    mse_kernel<<<grid_for(nout), 256, 0, s>>>(f->u, target, f->du, nout, f->lsum);
+    step_launch(mse_kernel, grid_for(nout), 256, 0, s, f->u, target, f->du, nout, f->lsum);
     FNO_CK(cudaGetLastError());
     // projection
     FNO_CK(weight_bias_grad((long long)rows, f->H, f->cout, f->h, f->H, f->du, f->cout,
@@ -1074,10 +1083,10 @@ int ehd_fno_adam_step(ehd_fno *f, float lr, float b1, float b2, float eps) {
     f->adam_t += 1;
     const float c1 = 1.f - std::pow(b1, (float)f->adam_t), c2 = 1.f - std::pow(b2, (float)f->adam_t);
     if (aligned16(f->param) && aligned16(f->grad) && aligned16(f->adam_m) && aligned16(f->adam_v))
-        adam4_kernel<<<grid_for(f->nparam / 4 + 1), 256, 0, f->stream>>>(
+        step_launch(adam4_kernel, grid_for(f->nparam / 4 + 1), 256, 0, f->stream, 
             f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
     else
-        adam_kernel<<<grid_for(f->nparam), 256, 0, f->stream>>>(
+        step_launch(adam_kernel, grid_for(f->nparam), 256, 0, f->stream, 
             f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
     FNO_CK(cudaGetLastError());
     FNO_CK(refresh(f));

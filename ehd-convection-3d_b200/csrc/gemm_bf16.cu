@@ -26,6 +26,7 @@
 #include <cstdint>
 #include <utility>
 
+#include "common.cuh"
 #include "gemm_bf16.cuh"
 
 namespace ehd {
@@ -129,6 +130,7 @@ __device__ __forceinline__ void row_offsets(Off (&ro)[16], unsigned &mask, const
 // instruction fetch.
 template <typename Off, int ABF, int AR, int BBF, int BR>
 __global__ void __launch_bounds__(128, 4) gemm_kernel(const GemmArgs a) {
+    step_enter();
     __shared__ __align__(16) __nv_bfloat16 As[BM][PK];
     __shared__ __align__(16) __nv_bfloat16 Bs[BN][PK];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -272,6 +274,7 @@ __device__ __forceinline__ void rw_load(float2 (&v)[KT][4], const float *A, int 
 template <int KT, int NT>
 __global__ void __launch_bounds__(256) rowwise_kernel(const GemmArgs a, int lda, int ldc,
                                                       int pair_store) {
+    step_enter();
     constexpr int PKB = 16 * KT + 8;  // padded row of B (BF16 elements)
     constexpr bool PF = KT <= 2;      // prefetch the next tile
     extern __shared__ __align__(16) unsigned char rw_smem[];
@@ -450,6 +453,7 @@ __device__ __forceinline__ void lm_epilogue(const GemmArgs &a, const float (&acc
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(256) leftmul_kernel(const GemmArgs a, int pair_store) {
+    step_enter();
     constexpr int NC = 8 * NT;
     extern __shared__ __align__(16) unsigned char lm_smem[];
     const int kt = (a.K + 15) / 16, KP = 16 * kt + 8;
@@ -560,6 +564,7 @@ constexpr int lm_stage_floats() { return 16 * (8 * NT + 4); }
 
 template <int MT, int NT>
 __global__ void __launch_bounds__(256) leftmul_cp_kernel(const GemmArgs a, int pair_store) {
+    step_enter();
     constexpr int NC = 8 * NT, RS = NC + 4, STAGE = lm_stage_floats<NT>();
     constexpr int C4 = NC / 4, CH = 16 * C4, CPL = (CH + 31) / 32;
     extern __shared__ __align__(16) unsigned char lm_smem[];
@@ -674,6 +679,7 @@ constexpr int SK_MAXK = 16, SK_MAXN = 128, SK_NJ = SK_MAXN / 32;
 
 template <int BF, int KK>
 __global__ void __launch_bounds__(256) smallk_kernel(const GemmArgs a) {
+    step_enter();
     __shared__ float As[8][32 * KK];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int N = a.N;
@@ -755,6 +761,7 @@ __global__ void __launch_bounds__(256, 2) wgrad_kernel(const float *__restrict__
                                                     const float *__restrict__ D, int ldd, int N,
                                                     long long rows, float *__restrict__ G,
                                                     int ldg, float *__restrict__ gb) {
+    step_enter();
     constexpr int NV = MT * NT * 128;         // partial sums of G per warp
     __shared__ float red[4][NV + NT * 8];     // warps w and w + 4 share a row
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -944,7 +951,7 @@ bool try_rowwise(const GemmArgs &a, cudaStream_t s, cudaError_t *err) {
     const long long want = (tiles + RW_WARPS - 1) / RW_WARPS;
     const long long per_batch = std::max(1ll, (long long)nsm * std::max(occ, 1) / a.batch);
     dim3 grid((unsigned)std::min(want, per_batch), (unsigned)a.batch, 1);
-    k<<<grid, 256, smem, s>>>(a, (int)a.am.s0, (int)a.cm.s0, pair);
+    step_launch(k, grid, 256, smem, s, a, (int)a.am.s0, (int)a.cm.s0, pair);
     *err = cudaGetLastError();
     return true;
 }
@@ -1041,7 +1048,7 @@ bool try_leftmul(const GemmArgs &a, cudaStream_t s, cudaError_t *err) {
     }
     const long long units = (long long)a.batch * ((a.N + 8 * nt - 1) / (8 * nt));
     const long long blocks = std::min((units + 7) / 8, (long long)nsm * std::max(occ, 1));
-    k<<<(unsigned)blocks, 256, smem, s>>>(a, pair ? 1 : 0);
+    step_launch(k, (unsigned)blocks, 256, smem, s, a, pair ? 1 : 0);
     *err = cudaGetLastError();
     return true;
 }
@@ -1077,7 +1084,7 @@ bool try_smallk(const GemmArgs &a, cudaStream_t s, cudaError_t *err) {
     // one wave of resident blocks, each warp walking its tiles
     const long long tiles = ((long long)a.M + 31) / 32;
     const long long blocks = std::min((tiles + 7) / 8, (long long)nsm * std::max(occ, 1));
-    k<<<(unsigned)blocks, 256, 0, s>>>(a);
+    step_launch(k, (unsigned)blocks, 256, 0, s, a);
     *err = cudaGetLastError();
     return true;
 }
@@ -1121,7 +1128,7 @@ cudaError_t weight_bias_grad(long long rows, int M, int N, const float *X, int l
             return e;
         const long long chunks = (rows + 15) / 16;
         const long long blocks = std::min((chunks + 7) / 8, (long long)nsm * std::max(occ, 1));
-        k<<<(unsigned)blocks, 256, 0, s>>>(X, ldx, M, D + n0, ldd, nn, rows, G + n0, ldg,
+        step_launch(k, (unsigned)blocks, 256, 0, s, X, ldx, M, D + n0, ldd, nn, rows, G + n0, ldg,
                                           gb ? gb + n0 : nullptr);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -1155,7 +1162,7 @@ cudaError_t gemm(const GemmArgs &a, cudaStream_t s) {
     const bool narrow = a.a_n < (1ll << 31) && a.b_n < (1ll << 31) && a.c_n < (1ll << 31);
     const int code = (narrow ? 16 : 0) | (a.a_bf16 ? 8 : 0) | (g.a_rows_fast ? 4 : 0) |
                      (a.b_bf16 ? 2 : 0) | (g.b_rows_fast ? 1 : 0);
-    kernel_table()[code]<<<grid, 128, 0, s>>>(g);
+    step_launch(kernel_table()[code], grid, 128, 0, s, g);
     return cudaGetLastError();
 }
 
