@@ -999,6 +999,14 @@ poisson_zdst_rt(typename Cplx<R>::T *__restrict__ spec, const typename Cplx<R>::
 // contiguous block.
 namespace {
 
+// transforms of a split-row block: those of 256 threads at once, but 16 (FP64:
+// 8) for N = 512, where those 4 would leave a block of NY = 512 (S = 8) a single
+// n, an 8-byte piece of each (j, kx) run of the split spectrum: the solve of
+// 512 x 512 x 129 in FP32 490 -> 368 us.
+template <typename R, int N> constexpr int split_block() {
+    return N == 512 ? (sizeof(R) == 8 ? 8 : 16) : per_block<N>();
+}
+
 // rows (ya, yb) of transform tr of a split-row block (two real rows per
 // complex transform): S = 1 pairs consecutive rows; S >= 2 pairs
 // n + 64 a and n + 64 (a + S/2) of group n = block * GB + tr / (S/2)
@@ -1041,6 +1049,27 @@ __device__ __forceinline__ R2 mul_ws(R2 x, int k) {
     return mul_w8(x, (k % S) * (8 / S));
 }
 
+// the block's TB transforms in place, a block barrier behind them: all at once,
+// or (N = 512) a warp each, in turns
+template <int N, int S, int TB, typename R2>
+__device__ __forceinline__ void split_transforms(R2 *buf, int stride, const R2 *tws) {
+    constexpr int G = fft::Plan<N>::G;
+    if constexpr (TB * G == 256) {
+        const int tr = threadIdx.x / G, j = threadIdx.x - tr * G;
+        fft::run_tile<N, S>(buf + tr * stride, tws, j);
+    } else {
+        static_assert(fft::WPlan<N>::G == 32 && TB % 8 == 0, "a warp per transform");
+#pragma unroll 1
+        for (int tr = threadIdx.x >> 5; tr < TB; tr += 8) {
+            R2 *b = buf + tr * stride;
+            fft::WPlan<N>::template run<S>(
+                b, tws, threadIdx.x & 31, [&](int m) { return b[fft::pad(m)]; },
+                [&](int m, R2 v) { b[fft::pad(m)] = v; });
+        }
+        __syncthreads();
+    }
+}
+
 // x-spectrum of row part (0: ya, 1: yb) of a packed transform at bin k < nxh
 template <typename R2, typename R>
 __device__ __forceinline__ R2 unpack_bin(const R2 *buf, int k, int part, int N) {
@@ -1071,7 +1100,7 @@ poisson_rows_fwd_split(const R *__restrict__ q, typename Cplx<R>::T *__restrict_
         qmean = (const double *)gp.qmean;
     }
     using R2 = typename Cplx<R>::T;
-    constexpr int G = fft::Plan<N>::G, TB = per_block<N>(), P = tstride<N>();
+    constexpr int TB = split_block<R, N>(), P = tstride<N>();
     constexpr int NY = 64 * S, GB = 2 * TB / S;
     static_assert(GB >= 1, "a block holds whole row groups");
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1140,10 +1169,7 @@ poisson_rows_fwd_split(const R *__restrict__ q, typename Cplx<R>::T *__restrict_
         split_rows<S, TB>(tid >> 1, ya, yb, g, a);
         rowsum[(size_t)zi * NY + ((tid & 1) ? yb : ya)] = -sum / eps;
     }
-    {
-        const int tr = tid / G, jj = tid - tr * G;
-        fft::run_tile<N, -1>(buf + tr * P, tws, jj);
-    }
+    split_transforms<N, -1, TB>(buf, P, tws);
     // items (g, kx), g fastest: the S rows n + 64 m of group g at bin kx, a
     // radix-S DFT over m, the twiddle W_NY^(j n), S outputs of GB consecutive
     // n per (j, kx)
@@ -1458,7 +1484,7 @@ poisson_rows_inv_split(const typename Cplx<R>::T *__restrict__ spl, R *__restric
         phip = (R *)gp.phip;
     }
     using R2 = typename Cplx<R>::T;
-    constexpr int G = fft::Plan<N>::G, TB = per_block<N>(), P = tstride<N>();
+    constexpr int TB = split_block<R, N>(), P = tstride<N>();
     constexpr int NY = 64 * S, GB = 2 * TB / S;
     constexpr int NB = S == 1 ? 2 * TB : GB;  // consecutive n per block
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1520,10 +1546,7 @@ poisson_rows_inv_split(const typename Cplx<R>::T *__restrict__ spl, R *__restric
         }
     }
     __syncthreads();
-    {
-        const int tr = tid / G, jj = tid - tr * G;
-        fft::run_tile<N, 1>(buf + tr * P, tws, jj);
-    }
+    split_transforms<N, 1, TB>(buf, P, tws);
     const R norm = (R)(1.0 / ((double)N * (double)NY));
     R *pp = phip + (size_t)N * NY * (zi + 1);
     for (int i = tid; i < TB * N; i += 256) {
@@ -1682,14 +1705,14 @@ static cudaError_t zdst(const PoissonArgs &a, cudaStream_t s) {
 
 template <typename R, int N, int S>
 constexpr size_t rows_inv_split_smem() {
-    constexpr int TB = per_block<N>();
+    constexpr int TB = split_block<R, N>();
     return sizeof(typename Cplx<R>::T) * ((size_t)N + (size_t)TB * tstride<N>());
 }
 
 template <typename R, int N, int S>
 static cudaError_t split_rows_fwd(const PoissonArgs &a, cudaStream_t s) {
     using R2 = typename Cplx<R>::T;
-    constexpr int TB = per_block<N>(), NB = S == 1 ? 2 * TB : 2 * TB / S;
+    constexpr int TB = split_block<R, N>(), NB = S == 1 ? 2 * TB : 2 * TB / S;
     const size_t sm = sizeof(R2) * ((size_t)N + (size_t)TB * tstride<N>());
     cudaError_t e = set_smem(poisson_rows_fwd_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
@@ -1701,7 +1724,7 @@ static cudaError_t split_rows_fwd(const PoissonArgs &a, cudaStream_t s) {
 template <typename R, int N, int S>
 static cudaError_t split_rows_inv(const PoissonArgs &a, cudaStream_t s) {
     using R2 = typename Cplx<R>::T;
-    constexpr int TB = per_block<N>(), NB = S == 1 ? 2 * TB : 2 * TB / S;
+    constexpr int TB = split_block<R, N>(), NB = S == 1 ? 2 * TB : 2 * TB / S;
     constexpr size_t sm = rows_inv_split_smem<R, N, S>();
     cudaError_t e = set_smem(poisson_rows_inv_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
