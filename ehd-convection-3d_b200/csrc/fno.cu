@@ -803,7 +803,8 @@ Dims dims(const ehd_fno *f, int B) {
         if (e_ != cudaSuccess) return cuda_fail(#call, e_); \
     } while (0)
 
-int forward(ehd_fno *f, int B, const float *a) {
+// keep: the hidden activations are kept for the backward pass
+int forward(ehd_fno *f, int B, const float *a, bool keep) {
     const Dims d = dims(f, B);
     const size_t rows = (size_t)B * f->P;
     const __nv_bfloat16 *pb = f->pbf;
@@ -825,6 +826,11 @@ int forward(ehd_fno *f, int B, const float *a) {
         FNO_CK(gemm(g, s));
     }
     const float *vL = f->z[f->L - 1];
+    if (!keep && project_usable((long long)rows, f->W, f->H, f->cout, vL)) {
+        FNO_CK(project((long long)rows, f->W, f->H, f->cout, vL, pb + f->oQ1, f->param + f->oq1,
+                       pb + f->oQ2, f->param + f->oq2, f->u, s));
+        return EHD_OK;
+    }
     FNO_CK(gemm(pointwise(rows, f->W, f->H, vL, pb + f->oQ1, f->hpre, f->param + f->oq1, f->h), s));
     FNO_CK(gemm(pointwise(rows, f->H, f->cout, f->h, pb + f->oQ2, f->u, f->param + f->oq2, nullptr),
                 s));
@@ -1011,7 +1017,7 @@ int ehd_fno_forward(ehd_fno *f, int B, const float *a, float *u) {
     if (!f || !a || !u) return fail("ehd_fno_forward: NULL argument");
     if (int r = check_batch(f, B)) return r;
     Dev dg(f->c.device);
-    if (int r = forward(f, B, a)) return r;
+    if (int r = forward(f, B, a, false)) return r;
     FNO_CK(cudaMemcpyAsync(u, f->u, (size_t)B * f->P * f->cout * sizeof(float),
                            cudaMemcpyDeviceToDevice, f->stream));
     return EHD_OK;
@@ -1022,7 +1028,7 @@ int ehd_fno_backward(ehd_fno *f, int B, const float *a, const float *target, dou
     if (int r = check_batch(f, B)) return r;
     Dev dg(f->c.device);
     cudaStream_t s = f->stream;
-    if (int r = forward(f, B, a)) return r;
+    if (int r = forward(f, B, a, true)) return r;
     const Dims d = dims(f, B);
     const size_t rows = (size_t)B * f->P;
     const size_t nout = rows * f->cout;

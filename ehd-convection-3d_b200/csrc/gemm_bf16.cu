@@ -365,6 +365,90 @@ __global__ void __launch_bounds__(256) rowwise_kernel(const GemmArgs a, int lda,
     }
 }
 
+// ---- the projection of a forward pass --------------------------------------
+//
+// u = gelu(A Q1 + q1) Q2 + q2 without the hidden activations in memory: a warp
+// forms 16 rows x 16 hidden columns, applies the GELU in registers and feeds
+// them, as the A fragment of the next K step, to the product with Q2 (the C
+// fragments of two 8-column tiles are laid out as that A fragment).  Rounding
+// and order of accumulation are those of the two rowwise products, so u is
+// the same bits.  The training pass keeps the two products, whose hidden
+// activations the backward pass reads.
+//
+// The two products moved 277 MB (pre-activation) + 2 x 277 MB (activation) at
+// 64 x 64 x 33, batch 4, in 256 us; this reads 69 and writes 11 MB and is bound
+// by the issue of the 69 M erff.
+template <int KT>
+__global__ void __launch_bounds__(256)
+project_kernel(const float *__restrict__ A, int M, int H, int cout,
+               const __nv_bfloat16 *__restrict__ Q1, const float *__restrict__ q1,
+               const __nv_bfloat16 *__restrict__ Q2, const float *__restrict__ q2,
+               float *__restrict__ u) {
+    step_enter();
+    constexpr int W = 16 * KT, PK1 = W + 8;
+    extern __shared__ __align__(16) unsigned char rw_smem[];
+    const int PK2 = H + 8;
+    __nv_bfloat16 *B1 = reinterpret_cast<__nv_bfloat16 *>(rw_smem);  // [H][PK1]
+    __nv_bfloat16 *B2 = B1 + H * PK1;                                // [8][PK2]
+    float *b1 = reinterpret_cast<float *>(B2 + 8 * PK2);             // [H]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gq = lane >> 2, tq = lane & 3;
+    for (int i = tid; i < W * H; i += 256) {
+        const int k = i / H, n = i - k * H;
+        B1[n * PK1 + k] = Q1[i];
+    }
+    for (int i = tid; i < 8 * H; i += 256) {
+        const int k = i >> 3, n = i & 7;
+        B2[n * PK2 + k] = n < cout ? Q2[k * cout + n] : __float2bfloat16_rn(0.f);
+    }
+    for (int i = tid; i < H; i += 256) b1[i] = q1[i];
+    __syncthreads();
+    const float o0 = 2 * tq < cout ? q2[2 * tq] : 0.f, o1 = 2 * tq + 1 < cout ? q2[2 * tq + 1] : 0.f;
+    const int tiles = (M + 15) / 16, tstride = gridDim.x * RW_WARPS;
+    int t = blockIdx.x * RW_WARPS + warp;
+    float2 cur[KT][4];
+    if (t < tiles) rw_load<KT>(cur, A, W, M, t, gq, tq);
+    for (; t < tiles; t += tstride) {
+        uint32_t af[KT][4];
+#pragma unroll
+        for (int s = 0; s < KT; ++s)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) af[s][e] = pack_bf16(cur[s][e]);
+        if (t + tstride < tiles) rw_load<KT>(cur, A, W, M, t + tstride, gq, tq);
+        float out[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+        for (int h0 = 0; h0 < H; h0 += 16) {
+            uint32_t ha[4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                const __nv_bfloat16 *bp = B1 + (h0 + 8 * j + gq) * PK1 + 2 * tq;
+#pragma unroll
+                for (int s = 0; s < KT; ++s) {
+                    const uint32_t w0 = *reinterpret_cast<const uint32_t *>(bp + 16 * s);
+                    const uint32_t w1 = *reinterpret_cast<const uint32_t *>(bp + 16 * s + 8);
+                    mma16816(acc, af[s][0], af[s][1], af[s][2], af[s][3], w0, w1);
+                }
+                const float2 b = *reinterpret_cast<const float2 *>(b1 + h0 + 8 * j + 2 * tq);
+                ha[2 * j] = pack_bf16(make_float2(gelu(acc[0] + b.x), gelu(acc[1] + b.y)));
+                ha[2 * j + 1] = pack_bf16(make_float2(gelu(acc[2] + b.x), gelu(acc[3] + b.y)));
+            }
+            const __nv_bfloat16 *cp = B2 + gq * PK2 + h0 + 2 * tq;
+            const uint32_t w0 = *reinterpret_cast<const uint32_t *>(cp);
+            const uint32_t w1 = *reinterpret_cast<const uint32_t *>(cp + 8);
+            mma16816(out, ha[0], ha[1], ha[2], ha[3], w0, w1);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = t * 16 + gq + 8 * h;
+            if (m >= M) continue;
+            float *row = u + (size_t)m * cout;
+            if (2 * tq < cout) row[2 * tq] = out[2 * h] + o0;
+            if (2 * tq + 1 < cout) row[2 * tq + 1] = out[2 * h + 1] + o1;
+        }
+    }
+}
+
 // ---- products by a small left matrix --------------------------------------
 //
 // For C[b][m][n] = alpha sum_k A[m][k] B[b][k][n] with one A for the whole
@@ -1164,6 +1248,26 @@ cudaError_t gemm(const GemmArgs &a, cudaStream_t s) {
                      (a.b_bf16 ? 2 : 0) | (g.b_rows_fast ? 1 : 0);
     step_launch(kernel_table()[code], grid, 128, 0, s, g);
     return cudaGetLastError();
+}
+
+// shapes whose two products run on the rowwise kernel, of up to 8 outputs
+bool project_usable(long long rows, int W, int H, int cout, const float *A) {
+    return (W == 16 || W == 32) && H % 16 == 0 && H <= 128 && cout <= 8 && rows < (1LL << 31) - 4096 &&
+           (reinterpret_cast<uintptr_t>(A) & 7) == 0;
+}
+cudaError_t project(long long rows, int W, int H, int cout, const float *A, const __nv_bfloat16 *Q1,
+                    const float *q1, const __nv_bfloat16 *Q2, const float *q2, float *u,
+                    cudaStream_t s) {
+    auto k = W == 16 ? project_kernel<1> : project_kernel<2>;
+    const size_t sm = sizeof(__nv_bfloat16) * ((size_t)H * (W + 8) + 8 * (size_t)(H + 8)) + sizeof(float) * H;
+    int occ = 0, dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, sm);
+    if (e != cudaSuccess) return e;
+    const long long tiles = (rows + 15) / 16;
+    const unsigned grid = (unsigned)std::min<long long>((tiles + RW_WARPS - 1) / RW_WARPS, (long long)nsm * occ);
+    return step_launch(k, grid, 256, sm, s, A, (int)rows, H, cout, Q1, q1, Q2, q2, u);
 }
 
 }  // namespace fno

@@ -79,5 +79,13 @@ cudaError_t gemm(const GemmArgs &a, cudaStream_t s);
 cudaError_t weight_bias_grad(long long rows, int M, int N, const float *X, int ldx, const float *D,
                              int ldd, float *G, int ldg, float *gb, cudaStream_t s);
 
+// u[rows][cout] = gelu(A[rows][W] Q1 + q1) Q2 + q2 in one kernel (Q1 [W][H], Q2
+// [H][cout] in BF16), the same bits as the two products; whether it serves a
+// shape
+bool project_usable(long long rows, int W, int H, int cout, const float *A);
+cudaError_t project(long long rows, int W, int H, int cout, const float *A, const __nv_bfloat16 *Q1,
+                    const float *q1, const __nv_bfloat16 *Q2, const float *q2, float *u,
+                    cudaStream_t s);
+
 }  // namespace fno
 }  // namespace ehd

@@ -145,3 +145,24 @@ def test_adam_training_fits_a_teacher_network():
             net.adam_step(lr=3e-3)
         last = net.backward(a, t)
     assert last < 0.1 * first, (first, last)
+
+
+@pytest.mark.parametrize("shape,batch,width,hidden,cout", [((17, 9, 5), 1, 16, 16, 1), ((16, 16, 8), 2, 32, 128, 5),
+                                                           ((19, 11, 7), 3, 32, 64, 8), ((8, 8, 4), 1, 16, 112, 3),
+                                                           ((18, 10, 6), 2, 32, 48, 7)])
+def test_forward_projection_is_the_two_products(shape, batch, width, hidden, cout):
+    """A forward pass projects in one kernel (hidden activations in registers),
+    a training pass by two products; the same arithmetic in the same order.
+    The loss of the training pass against the forward pass's output as its
+    target is then zero to the last bit: a batch whose rows end inside a tile,
+    the smallest and largest hidden widths, 1 to 8 outputs."""
+    import torch
+    nx, ny, nz = shape
+    net = fno.FNO(nx, ny, nz, 9, cout, width=width, layers=2, modes=(2, 2, 2), hidden=hidden,
+                  max_batch=batch, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(batch, nz, ny, nx, 9, device="cuda", generator=g)
+    u = net.forward(a)
+    assert torch.isfinite(u).all() and float(u.abs().max()) > 0
+    assert net.backward(a, u) == 0.0
+    net.close()
