@@ -207,11 +207,13 @@ __global__ void mix_kernel_w(const float *__restrict__ re, const float *__restri
 }
 
 // Gradient of R from the mixing's output gradient dout and its input x
-// (both Zh layout), added to gRe, gIm ([mode][out][in]):
-//   gRe[o][i] += sum_b dout_re[o] x_re[i] + dout_im[o] x_im[i]
-//   gIm[o][i] += sum_b dout_im[o] x_re[i] - dout_re[o] x_im[i]
+// (both Zh layout), into gRe, gIm ([mode][out][in]):
+//   gRe[o][i] = sum_b dout_re[o] x_re[i] + dout_im[o] x_im[i]
+//   gIm[o][i] = sum_b dout_im[o] x_re[i] - dout_re[o] x_im[i]
 // One warp per mode, both vectors of up to 4 samples staged in shared
-// memory, lanes along i (coalesced read-modify-write of the gradient rows).
+// memory, lanes along i.  The first samples' sums are written, not added to a
+// cleared gradient: the kernel is bound by the gradient's bytes (226 MB for
+// the four layers of 12^3 modes and 32 channels).
 __global__ void mix_wgrad_kernel(const float *__restrict__ dout, const float *__restrict__ x,
                                  float *__restrict__ gre, float *__restrict__ gim, int modes,
                                  int W, int B) {
@@ -233,14 +235,15 @@ __global__ void mix_wgrad_kernel(const float *__restrict__ dout, const float *__
                 X[t] = bb < nb ? __ldg(x + o) : 0.f;
             }
             __syncwarp();
-            // the gradient rows read eight at a time per lane, then updated
+            // the gradient rows eight at a time per lane
             for (int t0 = 0; t0 < W * W; t0 += 256) {
                 float og[8], om[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int t = t0 + 32 * u + lane;
-                    og[u] = t < W * W ? gr[t] : 0.f;
-                    om[u] = t < W * W ? gm[t] : 0.f;
+                    const bool add = b0 > 0 && t < W * W;
+                    og[u] = add ? gr[t] : 0.f;
+                    om[u] = add ? gm[t] : 0.f;
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -803,8 +806,9 @@ Dims dims(const ehd_fno *f, int B) {
         if (e_ != cudaSuccess) return cuda_fail(#call, e_); \
     } while (0)
 
-// keep: the hidden activations are kept for the backward pass
-int forward(ehd_fno *f, int B, const float *a, bool keep) {
+// u: the caller's output array (any alignment), or nullptr: the output goes to
+// f->u and the hidden activations are kept for the backward pass
+int forward(ehd_fno *f, int B, const float *a, float *u) {
     const Dims d = dims(f, B);
     const size_t rows = (size_t)B * f->P;
     const __nv_bfloat16 *pb = f->pbf;
@@ -826,14 +830,16 @@ int forward(ehd_fno *f, int B, const float *a, bool keep) {
         FNO_CK(gemm(g, s));
     }
     const float *vL = f->z[f->L - 1];
-    if (!keep && project_usable((long long)rows, f->W, f->H, f->cout, vL)) {
+    if (u && project_usable((long long)rows, f->W, f->H, f->cout, vL)) {
         FNO_CK(project((long long)rows, f->W, f->H, f->cout, vL, pb + f->oQ1, f->param + f->oq1,
-                       pb + f->oQ2, f->param + f->oq2, f->u, s));
+                       pb + f->oQ2, f->param + f->oq2, u, s));
         return EHD_OK;
     }
     FNO_CK(gemm(pointwise(rows, f->W, f->H, vL, pb + f->oQ1, f->hpre, f->param + f->oq1, f->h), s));
     FNO_CK(gemm(pointwise(rows, f->H, f->cout, f->h, pb + f->oQ2, f->u, f->param + f->oq2, nullptr),
                 s));
+    if (u)
+        FNO_CK(cudaMemcpyAsync(u, f->u, rows * f->cout * sizeof(float), cudaMemcpyDeviceToDevice, s));
     return EHD_OK;
 }
 
@@ -1017,9 +1023,7 @@ int ehd_fno_forward(ehd_fno *f, int B, const float *a, float *u) {
     if (!f || !a || !u) return fail("ehd_fno_forward: NULL argument");
     if (int r = check_batch(f, B)) return r;
     Dev dg(f->c.device);
-    if (int r = forward(f, B, a, false)) return r;
-    FNO_CK(cudaMemcpyAsync(u, f->u, (size_t)B * f->P * f->cout * sizeof(float),
-                           cudaMemcpyDeviceToDevice, f->stream));
+    if (int r = forward(f, B, a, u)) return r;
     return EHD_OK;
 }
 
@@ -1028,13 +1032,22 @@ int ehd_fno_backward(ehd_fno *f, int B, const float *a, const float *target, dou
     if (int r = check_batch(f, B)) return r;
     Dev dg(f->c.device);
     cudaStream_t s = f->stream;
-    if (int r = forward(f, B, a, true)) return r;
+    if (int r = forward(f, B, a, nullptr)) return r;
     const Dims d = dims(f, B);
     const size_t rows = (size_t)B * f->P;
     const size_t nout = rows * f->cout;
     float *g = f->grad;
     const __nv_bfloat16 *pb = f->pbf;
-    FNO_CK(cudaMemsetAsync(g, 0, f->nparam * sizeof(float), s));
+    {
+        // all gradients but the spectral weights' (mix_wgrad writes those)
+        const size_t spec = (size_t)f->modes * f->W * f->W;
+        size_t from = 0;
+        for (int l = 0; l <= f->L; ++l) {
+            const size_t to = l < f->L ? f->lo[l].Rre : f->nparam;
+            if (to > from) FNO_CK(cudaMemsetAsync(g + from, 0, (to - from) * sizeof(float), s));
+            if (l < f->L) from = f->lo[l].Rim + spec;
+        }
+    }
     FNO_CK(cudaMemsetAsync(f->lsum, 0, sizeof(double), s));
     step_launch(mse_kernel, grid_for(nout), 256, 0, s, f->u, target, f->du, nout, f->lsum);
     FNO_CK(cudaGetLastError());
