@@ -597,7 +597,7 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
         if ((r = dalloc(c, &c->ktab[i], c->rsize * 10 * nz))) return bail(r);
     }
     c->tune.lbm_kernel = (cfg.flags & EHD_FLAG_NODE_KERNEL) ? 1 : 0;
-    c->tune.node_block_x = lbm_default_block_x(nx);
+    c->tune.node_block_x = lbm_default_block_x(nx, c->prec == EHD_PREC_BF16);
     c->psum_blocks = lbm_blocks_per_plane(nx, ny, c->tune.node_block_x);
     {
         // the bulk-copy row kernel for steady-state steps, where it applies

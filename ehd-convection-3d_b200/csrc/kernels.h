@@ -101,7 +101,7 @@ cudaError_t launch_reduce_tables_group(const ReduceDesc *desc_dev, int n, int nz
 // psum slots per plane of the per-node kernel with blocks of bx x (128 / bx)
 int lbm_blocks_per_plane(int nx, int ny, int bx);
 // the per-node kernel's default block width for a grid nx wide
-int lbm_default_block_x(int nx);
+int lbm_default_block_x(int nx, bool bf16);
 // whether the bulk-copy row kernel serves this grid and storage type
 bool lbm_rows_usable(int nx, size_t fsize, size_t gsize);
 // sets the row kernel's shared-memory attribute (before any stream capture)

@@ -504,7 +504,7 @@ cudaError_t launch_lbm_step(const LbmArgs &la, const StepConst &c, int local_pop
         step_launch(rows_kernel<T, R>(macros, c.nx % 32 != 0), c.ny + la.rows_grid, tx, sm, s, a, k);
         return cudaGetLastError();
     }
-    const int bx = la.node_bx > 0 ? la.node_bx : lbm_default_block_x(c.nx);
+    const int bx = la.node_bx;
     dim3 block(bx, 128 / bx, 1);
     dim3 grid((c.nx + block.x - 1) / block.x, (c.ny + block.y - 1) / block.y, c.nz);
 #define EHD_LAUNCH(G, M) step_launch(lbm_step_kernel<T, R, G, M>, grid, block, 0, s, a, k, local_pops, e_arrays)
@@ -765,21 +765,29 @@ template cudaError_t launch_build_tables<float>(const double *, double *, const 
 template cudaError_t launch_build_tables<double>(const double *, double *, const double *,
                                                  void *, const StepConst &, cudaStream_t);
 
-// number of per-warp partial sums per plane written by the step kernel
-// the widest of 64, 32, 16 that leaves the fewest idle lanes at the row end
-// (96 -> 32, 80 and 48 -> 16, 256 and 122 -> 64)
-int lbm_default_block_x(int nx) {
-    int best = 64, waste = 1 << 30;
-    for (int bx : {64, 32, 16}) {
-        const int w = (nx + bx - 1) / bx * bx - nx;
-        if (w < waste) {
-            waste = w;
+// Block width of the per-node kernel: the least padded row, with a block 16
+// wide charged 15 % for its half-line accesses and wider ones 2 and 1 % less
+// than 32 (LBM half in us, 16 / 32 / 64 / 128 wide: 302 x 266 x 38 FP32 363 / 315 /
+// 302 / 311, 145^2 x 141 FP64 640 / 607 / 655 / 779, 122^2 x 101 FP32 182 / 157 / 153 /
+// 150, 271 x 255 x 30 mixed 235 / 209 / 222 / 251, 38^2 x 40 FP32 9.2 / 10.3 / 9.5 /
+// 12.1).  BF16 storage keeps the narrowest of the least padded of 64, 32 and
+// 16 (see keep_rt in api.cu: the width sets the order of the plane sums).
+int lbm_default_block_x(int nx, bool bf16) {
+    int best = 64;
+    double least = 1e30;
+    for (int bx : {64, 32, 16, 128}) {
+        if (bf16 && bx == 128) continue;
+        const double f = bf16 ? 1.0 : (bx == 16 ? 1.15 : (bx == 32 ? 1.02 : (bx == 64 ? 1.0 : 0.99)));
+        const double w = f * ((nx + bx - 1) / bx * bx);
+        if (w < least) {
+            least = w;
             best = bx;
         }
     }
     return best;
 }
 
+// number of per-warp partial sums per plane written by the per-node kernel
 int lbm_blocks_per_plane(int nx, int ny, int bx) {
     const int by = 128 / bx;
     return ((nx + bx - 1) / bx) * ((ny + by - 1) / by) * 4;
