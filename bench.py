@@ -40,10 +40,9 @@ ROOT = Path(__file__).resolve().parent
 PKG = ROOT / "ehd-convection-3d_b200"
 NX, NY, NZ = 256, 256, 129  # the workload; --grid overrides it for profiling only
 NODES = NX * NY * NZ
-# kernels per step of the FP32 256-wide workload: lbm_step (plane z = 0), lbm_rows
-# (planes z >= 1), reduce_tables, and the split-y Poisson's rows_fwd_split, slab,
-# rows_inv_split
-KERNELS_PER_STEP = 6
+# kernels per step of the FP32 256-wide workload: lbm_rows (with the plane z = 0),
+# reduce_tables, and the split-y Poisson's rows_fwd_split, slab, rows_inv_split
+KERNELS_PER_STEP = 5
 # Algorithmic bytes per node of one lbm_step launch (macros written, as
 # ehd_stream_collide_save does): 27 f + 27 g read and written, q written,
 # phi' read, rho/u/v/w written.  s = population bytes, p = field bytes.
@@ -54,7 +53,7 @@ def lbm_bytes_per_node(s: int, p: int) -> int:
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the LBM half
 # of one step on the full 256x256x129 grid, from an ncu capture of the row
 # kernel on the 256x256x33 grid (431.4 B per node), scaled to the 256x256x128
-# nodes the row kernel updates here, plus the z = 0 plane's launch.  A
+# nodes above z = 0, plus the z = 0 plane's own traffic.  A
 # recorded figure, not measured by this run; the line labels it so.
 NCU_TRAFFIC_BYTES = 3.66e9
 NCU_TRAFFIC_SOURCE = ("ncu capture of lbm_rows_kernel<float,float> at 256x256x33 "
@@ -395,8 +394,8 @@ def run_ours(args, rank, world, local_rank):
                 "how": "ehd_set_fields from pinned host memory, K x (ehd_step(1) + "
                        "ehd_current readback), ehd_get_fields to pinned host memory; wall clock"},
         "roofline": {"bound": "hbm",
-                     "kernel": "LBM half of the step: lbm_rows_kernel<float,float> (z >= 1) + "
-                               "lbm_step_kernel (z = 0) + plane-sum reduction and tables",
+                     "kernel": "LBM half of the step: lbm_rows_kernel<float,float> + "
+                               "plane-sum reduction and tables",
                      "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                      "bytes_per_node": lbm_bytes_per_node(4, 4),

@@ -385,9 +385,10 @@ size_t lbm_rows_smem(int nx, size_t fsize, size_t gsize) {
 }
 
 // FP32 and FP64 charge populations only: with both sets in 2 bytes the
-// per-node kernel measured faster (0.73 vs 0.76 ms at 256 x 256 x 129, FP16);
-// the mixed storage (2-byte f, 4-byte g) runs on it.  Rows are whole bulk
-// copies, so their bytes are multiples of 16.
+// per-node kernel measured faster (0.73 vs 0.76 ms at 256 x 256 x 129, FP16),
+// and lone FP16 and mixed contexts of an even NX step pairs (lbm_pair.cu).
+// The mixed storage (2-byte f, 4-byte g) runs on the rows in groups of a
+// batch.  Rows are whole bulk copies, so their bytes are multiples of 16.
 bool lbm_rows_usable(int nx, size_t fsize, size_t gsize) {
     return gsize >= 4 && nx >= 32 && nx <= 256 && (nx * fsize) % 16 == 0 &&
            (nx * gsize) % 16 == 0 && lbm_rows_smem(nx, fsize, gsize) <= 220 * 1024;

@@ -16,11 +16,14 @@
 //   K2 cols     : per plane, FFT along y of tiles of kx columns, in place; the
 //                 block of the first tile reduces the FP64 row sums to the
 //                 plane sum.
-//   K3 zsolve   : per (kx, ky) != (0,0), the tridiagonal system
+//   K3 z solve  : per (kx, ky) != (0,0), the tridiagonal system
 //                 phi(z-1) - (2 + k^2 dz^2) phi(z) + phi(z+1) = dz^2 s(z),
-//                 phi(0) = phi(NZ-1) = 0, by the Thomas algorithm in FP64
-//                 (pivots from a table built once per context, the forward
-//                 sweep in an FP64 scratch), in place.  The (0,0) mode in
+//                 phi(0) = phi(NZ-1) = 0, in place: as a sine transform where
+//                 2(NZ-1) is a compile-time FFT size (poisson_zdst) and in BF16
+//                 contexts (poisson_zdst_rt), otherwise eliminated from both
+//                 ends in FP64 (poisson_zmeet), or by a one-sided sweep with a
+//                 pivot table where the tuning asks for it (poisson_zsolve).
+//                 The (0,0) mode in
 //                 FP64 from the plane sums plus NX NY q_m, with the electrode
 //                 voltage entering as -V/dz^2 on the plane z = 1
 //                 (poisson.cu:97): the mean potential phi00(z) (V at z = 0)
@@ -32,11 +35,13 @@
 // phi = phi00(z) + phi'(x,y,z).  E = -grad(phi) is not stored: the step kernel
 // takes central differences of phi' and adds ez00(z), the mean-field Ez.
 //
-// FFTs: for N = 64, 128, 256, 512 the x and y transforms use compile-time
-// Stockham passes of radix 8/16 (fft.cuh), two real x-rows packed into one
-// complex transform; other sizes use run-time passes of radix 2/3/4/5 and,
+// FFTs: for N = 48, 64, 80, 96, 128, 256, 512 the x and y transforms use
+// compile-time Stockham passes (fft.cuh), two real x-rows packed into one
+// complex transform; other sizes are products with the folded DFT matrices
+// (dft.cu) or use run-time passes of radix 2/3/4/5 and,
 // for any other prime factor p, a direct radix-p pass over symmetric pairs
-// of outputs.  Twiddles come from an FP64-accurate table.
+// of outputs.  Twiddles come from an FP64-accurate table.  Where NY = 64 S,
+// K1..K4 are three kernels (the split-y path below).
 #include <cmath>
 
 #include "common.cuh"
