@@ -161,7 +161,7 @@ def build_case(name: str, nvcc: str = "nvcc") -> Path:
 
 
 def build(names=None) -> None:
-    if not REF_SRC.exists():
+    if not (REF_SRC / "LBM.h").exists():
         print("build_ref: reference sources absent; keeping prebuilt oracle/_ref")
         return
     names = list(names or CASES)
