@@ -237,7 +237,8 @@ int lbm(ehd_ctx *c, bool macros) {
     a.err = c->err;
     const int loc = c->pops_local ? 1 : 0, ea = c->e_arrays ? 1 : 0;
     const bool steady = c->tune.lbm_kernel == 0 && !loc && !ea;
-    const bool pair = c->pair && steady, rows = !pair && c->rows_grid > 0 && steady;
+    const bool pair = c->pair && steady;
+    const bool rows = c->prec == EHD_PREC_FP64 && c->rows_grid > 0 && steady;
     a.rows_grid = rows ? c->rows_grid : 0;
     a.node_bx = c->tune.node_block_x;
     cudaError_t e = cudaErrorInvalidValue;

@@ -22,7 +22,7 @@ struct LbmArgs {
     int node_bx;                    // per-node kernel block: node_bx x (128 / node_bx)
 };
 
-// ---- two nodes per thread, FP16 flow populations (csrc/lbm_pair.cu) ----
+// ---- two nodes per thread, FP32 and FP16 flow populations (csrc/lbm_pair.cu) ----
 // whether it serves a grid of n nodes (prec: ehd_precision); psum slots of a
 // plane z >= 1 (those of z = 0, twice as many, come first)
 bool lbm_pair_usable(int nx, long long n, int prec);

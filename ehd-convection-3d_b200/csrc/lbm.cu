@@ -50,7 +50,8 @@ lbm_step_kernel(const StepArgs<T, R> a, const KConst<R> c, int local_pops, int e
 
 // ---- bulk-copy row kernel ------------------------------------------------------
 
-// Persistent variant of the steady-state step for rows of NX nodes: one CTA
+// Persistent variant of the steady-state step for rows of NX nodes (FP64, and
+// FP32 and mixed storage in grouped launches): one CTA
 // of NX threads walks the x-rows (y, z) of the planes z >= 1, and the source
 // rows (y - e_y, z - e_z) of f_d and g_d of each row arrive in shared memory
 // by bulk copies, two rows ahead (two stages).  The x shift -e_x and its
@@ -249,6 +250,11 @@ lbm_rows_group_kernel(const LbmGroupDesc<T, R> *__restrict__ desc) {
     rows_cta<T, R, MACROS, PART>(sd.a, sd.k);
 }
 
+// A lone context steps rows in FP64 only: FP32 compute steps node pairs
+// (lbm_pair.cu), and has rows in the grouped launches alone.
+template <typename R>
+constexpr bool rows_alone() { return sizeof(R) == 8; }
+
 // the row kernels for (macro output, row ending inside a warp)
 template <typename T, typename R>
 using RowsKern = void (*)(const StepArgs<T, R>, const KConst<R>);
@@ -386,9 +392,10 @@ size_t lbm_rows_smem(int nx, size_t fsize, size_t gsize) {
 
 // FP32 and FP64 charge populations only: with both sets in 2 bytes the
 // per-node kernel measured faster (0.73 vs 0.76 ms at 256 x 256 x 129, FP16),
-// and lone FP16 and mixed contexts of an even NX step pairs (lbm_pair.cu).
-// The mixed storage (2-byte f, 4-byte g) runs on the rows in groups of a
-// batch.  Rows are whole bulk copies, so their bytes are multiples of 16.
+// and FP32 compute with an even NX steps pairs (lbm_pair.cu), so that rows
+// serve FP64 and, in the grouped launches of a batch, FP32 and mixed storage
+// (2-byte f, 4-byte g).  Rows are whole bulk copies, so their bytes are
+// multiples of 16.
 bool lbm_rows_usable(int nx, size_t fsize, size_t gsize) {
     return gsize >= 4 && nx >= 32 && nx <= 256 && (nx * fsize) % 16 == 0 &&
            (nx * gsize) % 16 == 0 && lbm_rows_smem(nx, fsize, gsize) <= 220 * 1024;
@@ -402,19 +409,22 @@ cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid) {
     if (!lbm_rows_usable(nx, sizeof(F), sizeof(G))) return cudaSuccess;
     const int sm = (int)lbm_rows_smem(nx, sizeof(F), sizeof(G));
     cudaError_t e;
-    for (int v = 0; v < 4; ++v)
-        if ((e = allow_max_dynamic_smem(rows_kernel<T, R>(v & 1, v & 2))) != cudaSuccess ||
-            (e = allow_max_dynamic_smem(rows_group_kernel<T, R>(v & 1, v & 2))) != cudaSuccess)
-            return e;
+    for (int v = 0; v < 4; ++v) {
+        if ((e = allow_max_dynamic_smem(rows_group_kernel<T, R>(v & 1, v & 2))) != cudaSuccess) return e;
+        if constexpr (rows_alone<R>())
+            if ((e = allow_max_dynamic_smem(rows_kernel<T, R>(v & 1, v & 2))) != cudaSuccess) return e;
+    }
     const bool part = nx % 32 != 0;
     int dev = 0, nsm = 0, occ_a = 0, occ_b = 0;
     const int tx = rows_block_x(nx);
+    auto kern = [&](bool macros) {
+        if constexpr (rows_alone<R>()) return rows_kernel<T, R>(macros, part);
+        else return rows_group_kernel<T, R>(macros, part);
+    };
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, rows_kernel<T, R>(true, part),
-                                                           tx, sm)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, rows_kernel<T, R>(false, part),
-                                                           tx, sm)) != cudaSuccess)
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_a, kern(true), tx, sm)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, kern(false), tx, sm)) != cudaSuccess)
         return e;
     const long long rows = (long long)ny * (nz - 1), slots = (long long)nsm * std::min(occ_a, occ_b);
     // where the injector plane's NY CTAs are few beside the resident ones,
@@ -498,12 +508,14 @@ cudaError_t launch_lbm_step(const LbmArgs &la, const StepConst &c, int local_pop
     StepArgs<T, R> a = make_step_args<T, R>(la, c);
     const KConst<R> k = make_kconst<R>(c);
     const bool general = local_pops || e_arrays;
-    if (!general && la.rows_grid > 0) {
-        // (its shared-memory attribute was set by prepare_lbm_rows)
-        const size_t sm = lbm_rows_smem(c.nx, sizeof(typename PopT<T>::F), sizeof(typename PopT<T>::G));
-        const int tx = rows_block_x(c.nx);
-        step_launch(rows_kernel<T, R>(macros, c.nx % 32 != 0), c.ny + la.rows_grid, tx, sm, s, a, k);
-        return cudaGetLastError();
+    if constexpr (rows_alone<R>()) {
+        if (!general && la.rows_grid > 0) {
+            // (its shared-memory attribute was set by prepare_lbm_rows)
+            const size_t sm = lbm_rows_smem(c.nx, sizeof(T), sizeof(T));
+            const int tx = rows_block_x(c.nx);
+            step_launch(rows_kernel<T, R>(macros, c.nx % 32 != 0), c.ny + la.rows_grid, tx, sm, s, a, k);
+            return cudaGetLastError();
+        }
     }
     const int bx = la.node_bx;
     dim3 block(bx, 128 / bx, 1);

@@ -1,5 +1,6 @@
-// lbm_pair.cu -- the steady-state step with two nodes per thread, for FP16
-// flow populations (FP16 and mixed storage) on grids of even NX.
+// lbm_pair.cu -- the steady-state step with two nodes per thread, for FP32
+// compute with FP32 or FP16 flow populations (FP32, FP16 and mixed storage) on
+// grids of even NX.
 //
 // With 2-byte populations the one-node-per-thread kernel is bound by the
 // issue of its instructions, not by memory: about 1,400 a node, at 512 x 512 x
@@ -18,9 +19,17 @@
 // 227 us for the LBM half.  What is left to the floor is load latency at that
 // occupancy (2.3 of 5.7 cycles between issues).
 //
+// FP32 populations are 64-bit words: 760 instructions a node and 128 loads of
+// a thread in flight, where the row kernel of lbm.cu spends about 1,340 and its
+// warps wait on whole rows.  LBM half of a step in us, the kernel it replaced /
+// this: 256 x 256 x 129 663 / 579 (6.66 TB/s of its 456 B a node, the copy
+// bandwidth), 128 x 128 x 65 96.5 / 80.8, 64 x 64 x 33 13.5 / 11.0, 200 x 200 x
+// 65 241 / 196 (rows); 122 x 122 x 101 148 / 113, 302 x 266 x 38 301 / 232,
+// 512 x 512 x 33 764 / 615, 38 x 38 x 40 9.2 / 7.7 (one node per thread).
+//
 // The injector plane z = 0 is stepped with one node per thread (node_step), by
-// blocks of the same launch on small grids, in a launch of its own on large
-// ones.  The pull, collision and wall rules are those of finish_node, on the
+// blocks of the same launch in FP32 and on small grids, in a launch of its own
+// on large ones.  The pull, collision and wall rules are those of finish_node, on the
 // same deviations.  (Rows through shared memory, as in lbm_rows_kernel, with
 // g read twice to stay at 128 registers, took 2.53 ms where this takes 2.15.)
 #include <type_traits>
@@ -331,17 +340,18 @@ int lbm_pair_slots(int nx, int ny) {
     return (pairs + kPairThreads - 1) / kPairThreads * (kPairThreads / 32);
 }
 
-// FP16 f with FP16 or FP32 g, rows of whole pairs, 32-bit byte offsets of the
-// 4-byte arrays
+// FP32, or FP16 f with FP16 or FP32 g; rows of whole pairs, 32-bit byte
+// offsets of the 4-byte arrays
 bool lbm_pair_usable(int nx, long long n, int prec) {
-    return (prec == 2 || prec == 4) && nx % 2 == 0 && n < (1LL << 30);
+    return (prec == 1 || prec == 2 || prec == 4) && nx % 2 == 0 && n < (1LL << 30);
 }
 
 // Up to so many blocks of pairs plane 0 goes with them: 64 x 64 x 33 in FP16
 // (512 blocks) 30.7 us a step with a launch of its own, 25.6 without, 100 x
 // 100 x 50 (2,000) 79.7 and 72.9; with many blocks the launch is nothing and the
 // kernel without the extra branch is the faster one: 256 x 256 x 129 (32,768)
-// 498 and 535.
+// 498 and 535.  In FP32 the branch costs nothing (122 x 122 x 101 160.6 us a
+// step with it, 164.9 without; 256 x 256 x 129 639.5 and 642.2): always merged.
 constexpr long long kMergeBlocks = 5000;
 
 template <typename T>
@@ -349,36 +359,39 @@ static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macro
     const StepArgs<T, float> a = make_step_args<T, float>(la, c);
     const KConst<float> k = make_kconst<float>(c);
     const int pairs = c.nx / 2 * c.ny, nb = (pairs + kPairThreads - 1) / kPairThreads;
-    if (nb * (long long)(c.nz - 1) <= kMergeBlocks) {
+    if (std::is_same<T, float>::value || nb * (long long)(c.nz - 1) <= kMergeBlocks) {
         const dim3 grid(nb, c.nz + 1);
         if (macros) step_launch(lbm_pair_kernel<T, true, StepArgs<T, float>>, grid, kPairThreads, 0, s, a, k);
         else step_launch(lbm_pair_kernel<T, false, StepArgs<T, float>>, grid, kPairThreads, 0, s, a, k);
         return cudaGetLastError();
     }
-    PairArgs<T> p;
-    p.pp = a.pp;
-    p.phip = a.phip;
-    p.ez00 = a.ez00;
-    p.qout = a.qout;
-    p.rout = a.rout;
-    p.uout = a.uout;
-    p.vout = a.vout;
-    p.wout = a.wout;
-    p.zref = a.zref;
-    p.psum = a.psum + 2 * lbm_pair_slots(c.nx, c.ny);
-    const dim3 grid(nb, c.nz - 1);
-    if (macros) {
-        step_launch(lbm_plane0_kernel<T, true>, 2 * nb, kPairThreads, 0, s, a, k);
-        step_launch(lbm_pair_kernel<T, true, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
-    } else {
-        step_launch(lbm_plane0_kernel<T, false>, 2 * nb, kPairThreads, 0, s, a, k);
-        step_launch(lbm_pair_kernel<T, false, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
+    if constexpr (!std::is_same<T, float>::value) {
+        PairArgs<T> p;
+        p.pp = a.pp;
+        p.phip = a.phip;
+        p.ez00 = a.ez00;
+        p.qout = a.qout;
+        p.rout = a.rout;
+        p.uout = a.uout;
+        p.vout = a.vout;
+        p.wout = a.wout;
+        p.zref = a.zref;
+        p.psum = a.psum + 2 * lbm_pair_slots(c.nx, c.ny);
+        const dim3 grid(nb, c.nz - 1);
+        if (macros) {
+            step_launch(lbm_plane0_kernel<T, true>, 2 * nb, kPairThreads, 0, s, a, k);
+            step_launch(lbm_pair_kernel<T, true, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
+        } else {
+            step_launch(lbm_plane0_kernel<T, false>, 2 * nb, kPairThreads, 0, s, a, k);
+            step_launch(lbm_pair_kernel<T, false, PairArgs<T>>, grid, kPairThreads, 0, s, p, k);
+        }
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_lbm_pair(int prec, const LbmArgs &la, const StepConst &c, bool macros,
                             cudaStream_t s) {
+    if (prec == 1) return pair_launch<float>(la, c, macros, s);
     return prec == 2 ? pair_launch<__half>(la, c, macros, s) : pair_launch<Mix16>(la, c, macros, s);
 }
 

@@ -88,7 +88,7 @@ typedef struct ehd_ctx ehd_ctx;
  * per-plane reference states, i.e. results at round-off level. */
 typedef struct ehd_tuning {
     int32_t lbm_kernel;      /* 0: steady steps on the kernel made for the grid
-                                and storage (columns; node pairs, FP16 f; rows)
+                                and storage (columns; node pairs, FP32 compute; rows)
                                 where one applies, else the per-node kernel;
                                 1: per-node                                   */
     int32_t node_block_x;    /* per-node kernel block: x extent 16, 32, 64 or

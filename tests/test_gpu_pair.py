@@ -1,12 +1,13 @@
-"""The two-nodes-per-thread step (csrc/lbm_pair.cu: FP16 and mixed storage, even
-nx) at the edges of its runs of node pairs: one pair a row, rows and planes
+"""The two-nodes-per-thread step (csrc/lbm_pair.cu: FP32, FP16 and mixed storage,
+even nx) at the edges of its runs of node pairs: one pair a row, rows and planes
 that end inside a warp and inside a block, the smallest stack, and the general
 sizes; against the oracle beside the per-node kernel.
 
-Both kernels round the same populations to FP16 once a step, at different
-places of the FP32 arithmetic, so their distances from the FP64 oracle have the
-same size: the pair kernel's is asked to be below twice the per-node kernel's
-(the spread between two realisations of the same rounding) plus 1e-6.
+Both kernels do the same FP32 arithmetic and round the same populations to their
+storage once a step, in a different order of operations, so their distances from
+the FP64 oracle have the same size: the pair kernel's is asked to be below twice
+the per-node kernel's (the spread between two realisations of the same rounding)
+plus 1e-6.
 """
 import numpy as np
 import pytest
@@ -18,7 +19,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("shape", [(2, 1, 4), (2, 5, 5), (6, 3, 4), (34, 3, 6), (64, 4, 5), (66, 7, 5),
                                    (128, 2, 6), (130, 9, 7), (256, 4, 5), (302, 5, 6)])
-@pytest.mark.parametrize("prec", ["fp16", "mixed"])
+@pytest.mark.parametrize("prec", ["fp16", "mixed", "fp32"])
 def test_pair_kernel_is_as_near_the_oracle_as_the_node_kernel(shape, prec):
     import make_golden as M
     nx, ny, nz = shape
