@@ -40,7 +40,7 @@ ROOT = Path(__file__).resolve().parent
 PKG = ROOT / "ehd-convection-3d_b200"
 NX, NY, NZ = 256, 256, 129  # the workload; --grid overrides it for profiling only
 NODES = NX * NY * NZ
-# kernels per step of the FP32 256-wide workload: lbm_rows (with the plane z = 0),
+# kernels per step of the FP32 256-wide workload: lbm_pair (with the plane z = 0),
 # reduce_tables, and the split-y Poisson's rows_fwd_split, slab, rows_inv_split
 KERNELS_PER_STEP = 5
 # Algorithmic bytes per node of one lbm_step launch (macros written, as
@@ -51,13 +51,13 @@ def lbm_bytes_per_node(s: int, p: int) -> int:
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the LBM half
-# of one step on the full 256x256x129 grid, from an ncu capture of the row
-# kernel on the 256x256x33 grid (431.4 B per node), scaled to the 256x256x128
+# of one step on the full 256x256x129 grid, from an ncu capture of the pair
+# kernel on the 256x256x33 grid (414.3 B per node), scaled to the 256x256x128
 # nodes above z = 0, plus the z = 0 plane's own traffic.  A
 # recorded figure, not measured by this run; the line labels it so.
-NCU_TRAFFIC_BYTES = 3.66e9
-NCU_TRAFFIC_SOURCE = ("ncu capture of lbm_rows_kernel<float,float> at 256x256x33 "
-                      "(431.4 B/node read+write), scaled by node count to 256x256x129")
+NCU_TRAFFIC_BYTES = 3.50e9
+NCU_TRAFFIC_SOURCE = ("ncu capture of lbm_pair_kernel<float> at 256x256x33 "
+                      "(414.3 B/node read+write), scaled by node count to 256x256x129")
 
 
 def reduce_max(x: float, dist=None, device="cpu") -> float:
@@ -394,7 +394,7 @@ def run_ours(args, rank, world, local_rank):
                 "how": "ehd_set_fields from pinned host memory, K x (ehd_step(1) + "
                        "ehd_current readback), ehd_get_fields to pinned host memory; wall clock"},
         "roofline": {"bound": "hbm",
-                     "kernel": "LBM half of the step: lbm_rows_kernel<float,float> + "
+                     "kernel": "LBM half of the step: lbm_pair_kernel<float> + "
                                "plane-sum reduction and tables",
                      "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
