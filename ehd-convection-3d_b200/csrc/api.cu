@@ -242,11 +242,10 @@ int lbm(ehd_ctx *c, bool macros) {
     a.rows_grid = rows ? c->rows_grid : 0;
     a.node_bx = c->tune.node_block_x;
     cudaError_t e = cudaErrorInvalidValue;
-    // psum slots: of plane 0, of the other planes
+    // psum slots per plane (psum_blocks follows the node kernel's block shape,
+    // see ehd_set_tuning)
     const int nblk = pair ? lbm_pair_slots(c->p.nx, c->p.ny)
                           : (rows ? lbm_rows_slots_per_plane(c->p.nx, c->p.ny) : c->psum_blocks);
-    const int nblk0 = pair ? 2 * nblk : nblk;
-    // (psum_blocks follows the node kernel's block shape, see ehd_set_tuning)
     if (pair) {
         e = launch_lbm_pair(c->prec, a, c->sc, macros, c->stream);
     } else switch (c->prec) {
@@ -262,8 +261,8 @@ int lbm(ehd_ctx *c, bool macros) {
     // now (the same phase of the injector's two-step alternation)
     const int p = c->cur;
     e = c->rsize == 8
-            ? launch_reduce_tables<double>(c->psum, c->mean[p ^ 1], nblk0, nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream)
-            : launch_reduce_tables<float>(c->psum, c->mean[p ^ 1], nblk0, nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream);
+            ? launch_reduce_tables<double>(c->psum, c->mean[p ^ 1], nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream)
+            : launch_reduce_tables<float>(c->psum, c->mean[p ^ 1], nblk, c->mean[p], c->wref[p], c->wref[p ^ 1], c->ktab[p ^ 1], c->sc, c->stream);
     if (e != cudaSuccess) return fail(EHD_ERR_CUDA, "reference tables: %s", cudaGetErrorString(e));
     c->cur ^= 1;
     c->pops_local = false;
@@ -495,7 +494,6 @@ int ctx_step_args(ehd_ctx *c, bool macros, LbmArgs *la, StepConst *sc, ReduceDes
     rd->nxy = c->sc.nxy;
     rd->nblk = rows ? lbm_rows_slots_per_plane(c->p.nx, c->p.ny)
                     : lbm_blocks_per_plane(c->p.nx, c->p.ny, c->tune.node_block_x);
-    rd->nblk0 = rd->nblk;
     rd->nz = c->p.nz;
     // poisson() after lbm() reads the plane means of the new state
     *pa = c->pa;
@@ -620,7 +618,7 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
         // room for the plane sums of every launch shape ehd_set_tuning allows
         c->pair = lbm_pair_usable(nx, c->sc.n, c->prec);
         int slots = c->rows_grid > 0 ? lbm_rows_slots_per_plane(nx, ny) : 0;
-        if (c->pair) slots = std::max(slots, 2 * lbm_pair_slots(nx, ny));
+        if (c->pair) slots = std::max(slots, lbm_pair_slots(nx, ny));
         for (int bx = 16; bx <= 128; bx *= 2) slots = std::max(slots, lbm_blocks_per_plane(nx, ny, bx));
         if ((r = dalloc(c, (void **)&c->psum, sizeof(float2) * (size_t)slots * nz))) return bail(r);
     }

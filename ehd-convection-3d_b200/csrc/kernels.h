@@ -23,8 +23,7 @@ struct LbmArgs {
 };
 
 // ---- two nodes per thread, FP32 and FP16 flow populations (csrc/lbm_pair.cu) ----
-// whether it serves a grid of n nodes (prec: ehd_precision); psum slots of a
-// plane z >= 1 (those of z = 0, twice as many, come first)
+// whether it serves a grid of n nodes (prec: ehd_precision); psum slots per plane
 bool lbm_pair_usable(int nx, long long n, int prec);
 int lbm_pair_slots(int nx, int ny);
 cudaError_t launch_lbm_pair(int prec, const LbmArgs &a, const StepConst &c, bool macros,
@@ -61,11 +60,10 @@ template <typename R>
 cudaError_t launch_build_tables(const double *msrc, double *wdst, const double *wread,
                                 void *ktab, const StepConst &c, cudaStream_t s);
 // psum_reduce and build_tables in one launch (the tables read msrc, the
-// previous means, so the two parts are independent); nblk0 slots of plane 0,
-// then nblk of each other plane
+// previous means, so the two parts are independent)
 template <typename R>
-cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk0, int nblk,
-                                 const double *msrc, double *wdst, const double *wread, void *ktab,
+cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk, const double *msrc,
+                                 double *wdst, const double *wread, void *ktab,
                                  const StepConst &c, cudaStream_t s);
 // ---- launches over a group of instances with the same grid ----------------
 // (batch steps, csrc/batch.cu): one launch per kernel covers every instance.
@@ -93,7 +91,7 @@ struct ReduceDesc {
     const double *wread;
     void *ktab;
     long long nxy;
-    int nblk0, nblk, nz;
+    int nblk, nz;
 };
 template <typename R>
 cudaError_t launch_reduce_tables_group(const ReduceDesc *desc_dev, int n, int nz, cudaStream_t s);

@@ -643,18 +643,15 @@ __global__ void fields_plane_mean_kernel(const double *__restrict__ rho,
 }
 
 // Plane means from the step kernel's per-block sums (fixed order).
-// Plane z's sums of rho and q over its per-warp slots (nblk0 of plane 0, then
-// nblk of each other plane), as means, into m[2z], m[2z+1]; fixed summation
-// order.  One block of 256 threads.
+// Plane z's sums of rho and q over its nblk slots, as means, into m[2z],
+// m[2z+1]; fixed summation order.  One block of 256 threads.
 __device__ __forceinline__ void psum_reduce_block(const float2 *__restrict__ psum,
-                                                  double *__restrict__ m, int nblk0, int nblk,
-                                                  long long nxy, int z) {
-    if (z == 0) nblk = nblk0;
-    else psum += nblk0 + (size_t)(z - 1) * nblk;
+                                                  double *__restrict__ m, int nblk, long long nxy,
+                                                  int z) {
     __shared__ double wr[8], wq[8];
     double a = 0.0, b = 0.0;
     for (int i = threadIdx.x; i < nblk; i += 256) {
-        const float2 v = psum[i];
+        const float2 v = psum[(size_t)z * nblk + i];
         a += v.x;
         b += v.y;
     }
@@ -721,11 +718,11 @@ __global__ void build_tables_kernel(const double *__restrict__ msrc, double *wds
 // the previous means, not the ones reduced here).  One launch per step.
 template <typename R>
 __global__ void __launch_bounds__(256)
-reduce_tables_kernel(const float2 *__restrict__ psum, double *__restrict__ m, int nblk0, int nblk,
+reduce_tables_kernel(const float2 *__restrict__ psum, double *__restrict__ m, int nblk,
                      long long nxy, const double *__restrict__ msrc, double *wdst,
                      const double *wread, R *__restrict__ ktab, int nz) {
     step_enter();
-    if ((int)blockIdx.x < nz) psum_reduce_block(psum, m, nblk0, nblk, nxy, blockIdx.x);
+    if ((int)blockIdx.x < nz) psum_reduce_block(psum, m, nblk, nxy, blockIdx.x);
     else build_tables_block<R>(msrc, wdst, wread, ktab, nz);
 }
 
@@ -735,7 +732,7 @@ template <typename R>
 __global__ void __launch_bounds__(256)
 reduce_tables_group_kernel(const ReduceDesc *__restrict__ desc) {
     const ReduceDesc &r = desc[blockIdx.y];
-    if ((int)blockIdx.x < r.nz) psum_reduce_block(r.psum, r.m, r.nblk0, r.nblk, r.nxy, blockIdx.x);
+    if ((int)blockIdx.x < r.nz) psum_reduce_block(r.psum, r.m, r.nblk, r.nxy, blockIdx.x);
     else build_tables_block<R>(r.msrc, r.wdst, r.wread, (R *)r.ktab, r.nz);
 }
 template <typename R>
@@ -760,19 +757,19 @@ cudaError_t launch_build_tables(const double *msrc, double *wdst, const double *
     return cudaGetLastError();
 }
 template <typename R>
-cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk0, int nblk,
-                                 const double *msrc, double *wdst, const double *wread,
-                                 void *ktab, const StepConst &c, cudaStream_t s) {
-    step_launch(reduce_tables_kernel<R>, c.nz + 1, 256, 0, s, psum, m, nblk0, nblk, c.nxy, msrc, wdst, wread,
-                                                     (R *)ktab, c.nz);
+cudaError_t launch_reduce_tables(const float2 *psum, double *m, int nblk, const double *msrc,
+                                 double *wdst, const double *wread, void *ktab,
+                                 const StepConst &c, cudaStream_t s) {
+    step_launch(reduce_tables_kernel<R>, c.nz + 1, 256, 0, s, psum, m, nblk, c.nxy, msrc, wdst,
+                wread, (R *)ktab, c.nz);
     return cudaGetLastError();
 }
-template cudaError_t launch_reduce_tables<float>(const float2 *, double *, int, int,
-                                                 const double *, double *, const double *,
-                                                 void *, const StepConst &, cudaStream_t);
-template cudaError_t launch_reduce_tables<double>(const float2 *, double *, int, int,
-                                                  const double *, double *, const double *,
-                                                  void *, const StepConst &, cudaStream_t);
+template cudaError_t launch_reduce_tables<float>(const float2 *, double *, int, const double *,
+                                                 double *, const double *, void *,
+                                                 const StepConst &, cudaStream_t);
+template cudaError_t launch_reduce_tables<double>(const float2 *, double *, int, const double *,
+                                                  double *, const double *, void *,
+                                                  const StepConst &, cudaStream_t);
 template cudaError_t launch_build_tables<float>(const double *, double *, const double *, void *,
                                                 const StepConst &, cudaStream_t);
 template cudaError_t launch_build_tables<double>(const double *, double *, const double *,

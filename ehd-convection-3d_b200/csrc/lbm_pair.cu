@@ -99,10 +99,11 @@ struct PairArgs {
     const double *ez00;
     float *qout, *rout, *uout, *vout, *wout;
     const float *zref;
-    float2 *psum;  // slots of the planes z >= 1: [z - 1][warp]
+    float2 *psum;  // [z][block][8]
 };
 
-// Block b of plane 0, one node per thread; its plane sums come first.
+// Block b of plane 0, one node per thread: two of them fill the eight plane-sum
+// slots of a block of pairs.
 template <typename T, bool MACROS>
 __device__ __forceinline__ void plane0_block(const StepArgs<T, float> &a, const KConst<float> &c,
                                              int b) {
@@ -171,11 +172,30 @@ lbm_pair_kernel(const Args a, const KConst<float> c) {
         f[d] = pull(a.pp.fa[d], r + xm, r + x0, r + xq, ex_of(d));
         h[d] = pull(a.pp.ha[d], r + xm, r + x0, r + xq, ex_of(d));
     }
+    // To this step's references, in one rounding as in pull_global: w times the
+    // shift, rounded before it is added, would be off by the same amount at every
+    // node of a plane (FP32, 64 x 64 x 33, 100 steps, 24 starts: distance of u and
+    // phi from the 64-bit run 1.012 and 1.006 times the per-node kernel's, 1.000
+    // and 1.001 so).  256 x 256 x 129 in FP32 643 us a step, 640 with the rounded
+    // products; 122 x 122 x 101 167 and 161.  16-bit f direction by direction of e_z, which leaves the kernel
+    // registers for more loads: FP16 499 us, in the order of d 508.
+    auto shift = [&](int d) {
+        const float2 w = dup(c.w[cls_of(d)]);
+        f[d] = fma2(w, dup(ez_of(d) > 0 ? zr[2] : (ez_of(d) < 0 ? zr[4] : zr[3])), f[d]);
+        h[d] = fma2(w, dup(ez_of(d) > 0 ? zr[5] : (ez_of(d) < 0 ? zr[7] : zr[6])), h[d]);
+    };
+    if constexpr (std::is_same<T, float>::value) {
+#pragma unroll
+        for (int d = 0; d < Q; ++d) shift(d);
+    } else {
+#pragma unroll
+        for (int e = -1; e <= 1; ++e)
+#pragma unroll
+            for (int d = 0; d < Q; ++d)
+                if (ez_of(d) == e) shift(d);
+    }
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
-        const float w = c.w[cls_of(d)];
-        f[d] = add2(f[d], dup(w * (ez_of(d) > 0 ? zr[2] : (ez_of(d) < 0 ? zr[4] : zr[3]))));
-        h[d] = add2(h[d], dup(w * (ez_of(d) > 0 ? zr[5] : (ez_of(d) < 0 ? zr[7] : zr[6]))));
         drho = add2(drho, f[d]);
         dq = add2(dq, h[d]);
         if (ex_of(d)) mx = ex_of(d) > 0 ? add2(mx, f[d]) : fma2(mone, f[d], mx);
@@ -184,15 +204,17 @@ lbm_pair_kernel(const Args a, const KConst<float> c) {
     }
     const float2 rho = add2(dup(zr[0]), drho), charge = add2(dup(zr[1]), dq);
     {
+        // FP32 sums of 32 nodes, as in the other step kernels: each half of the
+        // warp has a slot
         float2 v = make_float2(inside ? rho.x + rho.y : 0.f, inside ? charge.x + charge.y : 0.f);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = 8; o > 0; o >>= 1) {
             v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
             v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
-        if ((threadIdx.x & 31) == 0)
-            a.psum[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (kPairThreads / 32) +
-                   (threadIdx.x >> 5)] = v;
+        if ((threadIdx.x & 15) == 0)
+            a.psum[((size_t)z * gridDim.x + blockIdx.x) * (kPairThreads / 16) +
+                   (threadIdx.x >> 4)] = v;
     }
     if (!inside) return;
 
@@ -334,10 +356,9 @@ lbm_pair_kernel(const Args a, const KConst<float> c) {
     }
 }
 
-// psum slots of a plane z >= 1 (plane 0: twice as many)
 int lbm_pair_slots(int nx, int ny) {
     const int pairs = nx / 2 * ny;
-    return (pairs + kPairThreads - 1) / kPairThreads * (kPairThreads / 32);
+    return (pairs + kPairThreads - 1) / kPairThreads * (kPairThreads / 16);
 }
 
 // FP32, or FP16 f with FP16 or FP32 g; rows of whole pairs, 32-bit byte
@@ -376,7 +397,7 @@ static cudaError_t pair_launch(const LbmArgs &la, const StepConst &c, bool macro
         p.vout = a.vout;
         p.wout = a.wout;
         p.zref = a.zref;
-        p.psum = a.psum + 2 * lbm_pair_slots(c.nx, c.ny);
+        p.psum = a.psum;
         const dim3 grid(nb, c.nz - 1);
         if (macros) {
             step_launch(lbm_plane0_kernel<T, true>, 2 * nb, kPairThreads, 0, s, a, k);
