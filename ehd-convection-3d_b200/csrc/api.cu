@@ -669,12 +669,16 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     const bool keep_rt = c->prec == EHD_PREC_BF16;
     // z solve: the sine transform where 2 (nz - 1) is a compile-time FFT size;
     // elsewhere the Thomas solves, with their pivot table and the FP64 sweep's
-    // scratch (ehd_tuning.z_solve)
+    // scratch (ehd_tuning.z_solve).  Columns too tall for the two-sided solve's
+    // shared memory take the sine transform with run-time passes while that
+    // fits, NZ up to 1463 in FP64 and 2560 in FP32 (step in us, so / with the
+    // FP64 sweep: 64 x 64 x 901 FP64 977 / 1560, 16 x 16 x 1401 FP64 314 / 1484,
+    // 64 x 64 x 2001 FP32 1428 / 3115).
     const int lz2 = 2 * (nz - 1);
     const bool thomas = !poisson_fast_size(lz2);
     bool zdst = !thomas;
     pa.ztb = 0;
-    if (thomas && keep_rt) {
+    if (thomas && (keep_rt || zmeet_modes(nz, c->rsize) == 0)) {
         int tb = 16;
         while (tb > 1 && zdst_rt_smem(lz2, tb, c->rsize) > 160 * 1024) tb >>= 1;
         if (zdst_rt_smem(lz2, tb, c->rsize) <= 160 * 1024) {

@@ -102,9 +102,10 @@ typedef struct ehd_tuning {
                                 else the five-kernel one; 1: five-kernel     */
     int32_t z_solve;         /* where 2 (NZ-1) is not a compile-time FFT
                                 size (48, 64, 80, 96, 128, 256, 512): 0 the
-                                two-sided Thomas solve in shared memory (where
-                                a column fits; BF16 storage: the sine transform
-                                with run-time passes), 1 the FP64 Thomas sweep */
+                                two-sided Thomas solve in shared memory (BF16
+                                storage, and columns too tall for that: the
+                                sine transform with run-time passes, while it
+                                fits), 1 the FP64 Thomas sweep                */
     int32_t reserved[2];     /* must be 0                                     */
 } ehd_tuning;
 
