@@ -530,6 +530,62 @@ dft_cols(const typename Cplx<R>::T *__restrict__ in, typename Cplx<R>::T *__rest
     }
 }
 
+namespace {
+// The mean mode of a tall column, x_i = -((n + 1 - i) A_i + i B_i) / (n + 1) / nxy
+// with A_i = sum_{j < i} j rhs_j and B_i = sum_{j >= i} (n + 1 - j) rhs_j (i, j = 1..n),
+// by the block of 128 threads: a run of planes each, the sums before and after
+// it from one scan.  The n terms of every plane, each a dependent FP64 step, would
+// be the solve's longest chain: 4 x 4 x 1729 in FP32 288 us a step with them,
+// @@ so; below kTallMean planes they hide behind the modes.
+constexpr int kTallMean = 512;
+__device__ __noinline__ void tall_mean(const double *mrhs, double *mphi, double *phi00, int nz,
+                                       double nxy, double voltage) {
+    // (not static shared memory: the columns of the other blocks would move off
+    // their 128-byte lines)
+    double *wa = mphi + nz, *wb = wa + 4;
+    const int n = nz - 2, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c = (n + 127) / 128;
+    const int i0 = 1 + tid * c < n + 1 ? 1 + tid * c : n + 1, i1 = i0 + c < n + 1 ? i0 + c : n + 1;
+    double a = 0.0, b = 0.0;
+    for (int i = i0; i < i1; ++i) {
+        a += (double)i * mrhs[i - 1];
+        b += (double)(n + 1 - i) * mrhs[i - 1];
+    }
+    // sums of a over the threads before, of b over those after
+    double sa = a, sb = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double ta = __shfl_up_sync(0xffffffffu, sa, o), tb = __shfl_down_sync(0xffffffffu, sb, o);
+        if (lane >= o) sa += ta;
+        if (lane + o < 32) sb += tb;
+    }
+    if (lane == 31) wa[warp] = sa;
+    if (lane == 0) wb[warp] = sb;
+    double A = __shfl_up_sync(0xffffffffu, sa, 1), B = __shfl_down_sync(0xffffffffu, sb, 1);
+    if (lane == 0) A = 0.0;
+    if (lane == 31) B = 0.0;
+    __syncthreads();
+    for (int w = 0; w < 4; ++w) {
+        if (w < warp) A += wa[w];
+        if (w > warp) B += wb[w];
+    }
+    for (int i = i0; i < i1; ++i) {
+        mphi[i] = (double)(n + 1 - i) * A;
+        A += (double)i * mrhs[i - 1];
+    }
+    for (int i = i1 - 1; i >= i0; --i) {
+        B += (double)(n + 1 - i) * mrhs[i - 1];
+        const double x = -(mphi[i] + (double)i * B) / (double)(n + 1) / nxy;
+        mphi[i] = x;
+        phi00[i] = x;
+    }
+    if (tid == 0) {
+        mphi[0] = phi00[0] = voltage;
+        mphi[nz - 1] = phi00[nz - 1] = 0.0;
+    }
+}
+}  // namespace
+
 // K3 for any NZ whose columns fit in shared memory: the tridiagonal system of
 // poisson_zsolve per mode (kx, ky), phi(z-1) - beta phi(z) + phi(z+1) =
 // dz^2 s(z), beta = 2 + (kx^2 + ky^2) dz^2, phi = 0 on the electrodes, solved
@@ -546,7 +602,7 @@ dft_cols(const typename Cplx<R>::T *__restrict__ in, typename Cplx<R>::T *__rest
 // mode in closed form beside the others (see poisson_zdst); the (0,0) mode of
 // the fluctuation is 0.
 template <typename R>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 2)
 poisson_zmeet(typename Cplx<R>::T *__restrict__ spec, const double *__restrict__ cpt,
               const double *__restrict__ planesum, const double *__restrict__ qmean,
               double *__restrict__ phi00, double *__restrict__ ez00, int nx, int ny, int nz,
@@ -575,7 +631,9 @@ poisson_zmeet(typename Cplx<R>::T *__restrict__ spec, const double *__restrict__
             mrhs[i] = d * dz2;
         }
         __syncthreads();
-        for (int i = tid; i < nz; i += 128) {
+        if (nz > kTallMean) {
+            tall_mean(mrhs, mphi, phi00, nz, nxy, voltage);
+        } else for (int i = tid; i < nz; i += 128) {
             double x = 0.0;
             if (i == 0) {
                 x = voltage;
@@ -617,6 +675,17 @@ poisson_zmeet(typename Cplx<R>::T *__restrict__ spec, const double *__restrict__
                              "l"(g + (size_t)z * plane)
                              : "memory");
         }
+    // the block's pivots into L2, by 32-byte pieces: where the state is larger
+    // than L2 they are gone from one step to the next, and the chain would wait
+    // for each batch of them
+    {
+        const int per = mb / 4 + 1;
+        for (int i = tid; i < (n / 2) * per; i += 128) {
+            const int k = i / per, m = m0 + 4 * (i - k * per);
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                cpt + (size_t)k * modes + (m < modes ? m : modes - 1)));
+        }
+    }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     if (16 * warp < mb) {
@@ -891,8 +960,9 @@ template <typename R>
 cudaError_t launch_zmeet(const PoissonArgs &a, cudaStream_t s) {
     using R2 = typename Cplx<R>::T;
     const int mb = zmeet_modes(a.nz, sizeof(R)), modes = a.nxh * a.ny;
-    // (at least the mean mode's two FP64 arrays)
-    const size_t cols = sizeof(R2) * (size_t)mb * (a.nz - 2), mean = sizeof(double) * 2 * (size_t)a.nz;
+    // (at least the mean mode's two FP64 arrays and partial sums)
+    const size_t cols = sizeof(R2) * (size_t)mb * (a.nz - 2),
+                 mean = sizeof(double) * (2 * (size_t)a.nz + 8);
     const size_t sm = cols > mean ? cols : mean;
     cudaError_t e = set_smem(poisson_zmeet<R>, sm, s);
     if (e != cudaSuccess) return e;
