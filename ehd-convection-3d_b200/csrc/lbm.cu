@@ -427,9 +427,15 @@ cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid) {
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, kern(false), tx, sm)) != cudaSuccess)
         return e;
     const long long rows = (long long)ny * (nz - 1), slots = (long long)nsm * std::min(occ_a, occ_b);
-    // where the injector plane's NY CTAs are few beside the resident ones,
-    // they get their slots, so that no row waits for them
-    *grid = (int)std::min<long long>(rows, ny <= slots / 4 ? slots - ny : slots);
+    // The injector plane's NY CTAs get slots of their own, so that no row waits
+    // for them, where that makes no CTA's run of rows longer; otherwise rows take
+    // every slot, and some start a row or two late.  LBM half in us with own slots
+    // / without, FP64: 256 x 16 x 33 (4 rows a CTA either way) 25.9 / 27.5; 200 x
+    // 30 x 17 (5 or 4) 26.6 / 24.6, 128 x 32 x 65 (8 or 7) 51.0 / 48.2, 128 x 64 x 129
+    // (36 or 28) 179 / 165, 96 x 40 x 401 (63 or 55) 290 / 261.
+    auto run = [&](long long n) { return (rows + n - 1) / n; };
+    const bool own = ny < slots && run(slots - ny) == run(slots);
+    *grid = (int)std::min<long long>(rows, own ? slots - ny : slots);
     return cudaSuccess;
 }
 
