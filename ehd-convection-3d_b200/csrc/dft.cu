@@ -535,8 +535,8 @@ namespace {
 // with A_i = sum_{j < i} j rhs_j and B_i = sum_{j >= i} (n + 1 - j) rhs_j (i, j = 1..n),
 // by the block of 128 threads: a run of planes each, the sums before and after
 // it from one scan.  The n terms of every plane, each a dependent FP64 step, would
-// be the solve's longest chain: 4 x 4 x 1729 in FP32 288 us a step with them,
-// @@ so; below kTallMean planes they hide behind the modes.
+// be the solve's longest chain: 4 x 4 x 1729 in FP32 287 us a step with them,
+// 208 so; up to kTallMean planes they hide behind the modes.
 constexpr int kTallMean = 512;
 __device__ __noinline__ void tall_mean(const double *mrhs, double *mphi, double *phi00, int nz,
                                        double nxy, double voltage) {
@@ -600,7 +600,9 @@ __device__ __noinline__ void tall_mean(const double *mrhs, double *mphi, double 
 // small blocks, whose columns arrive (cp.async, every load in flight at once)
 // and leave while others' chains run.  Block 0 solves the (0,0)
 // mode in closed form beside the others (see poisson_zdst); the (0,0) mode of
-// the fluctuation is 0.
+// the fluctuation is 0.  The bound of two blocks a multiprocessor leaves the
+// compiler registers for whole batches of loads (FP64 90 instead of 72: 16 x 16 x
+// 865 194 -> 180 us a step).
 template <typename R>
 __global__ void __launch_bounds__(128, 2)
 poisson_zmeet(typename Cplx<R>::T *__restrict__ spec, const double *__restrict__ cpt,
@@ -677,7 +679,7 @@ poisson_zmeet(typename Cplx<R>::T *__restrict__ spec, const double *__restrict__
         }
     // the block's pivots into L2, by 32-byte pieces: where the state is larger
     // than L2 they are gone from one step to the next, and the chain would wait
-    // for each batch of them
+    // for each batch of them (16 x 16 x 865 in FP64 203 -> 194 us a step)
     {
         const int per = mb / 4 + 1;
         for (int i = tid; i < (n / 2) * per; i += 128) {
