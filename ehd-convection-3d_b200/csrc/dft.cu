@@ -883,6 +883,11 @@ cudaError_t with_tile(int n, int unit, F f) {
 }  // namespace
 
 template <typename R>
+cudaError_t prepare_zmeet() {
+    return allow_max_dynamic_smem(poisson_zmeet<R>);
+}
+
+template <typename R>
 cudaError_t prepare_dft(int nx, int ny) {
     cudaError_t e = with_tile<R>(nx, kXU, [&](auto tn, auto even) {
         cudaError_t r = allow_max_dynamic_smem(dft_rows_fwd<R, decltype(tn)::value, decltype(even)::value>);
@@ -897,8 +902,7 @@ cudaError_t prepare_dft(int nx, int ny) {
                        ? allow_max_dynamic_smem(dft_cols<R, 1, decltype(tn)::value, decltype(even)::value>)
                        : r;
         });
-    if (e == cudaSuccess) e = allow_max_dynamic_smem(poisson_zmeet<R>);
-    return e;
+    return e == cudaSuccess ? prepare_zmeet<R>() : e;
 }
 
 template <typename R>
@@ -976,6 +980,7 @@ cudaError_t launch_zmeet(const PoissonArgs &a, cudaStream_t s) {
 }
 
 #define EHD_INST_DFT(R)                                                       \
+    template cudaError_t prepare_zmeet<R>();                                 \
     template cudaError_t prepare_dft<R>(int, int);                           \
     template cudaError_t launch_dft_rows_fwd<R>(const PoissonArgs &, cudaStream_t); \
     template cudaError_t launch_dft_rows_inv<R>(const PoissonArgs &, cudaStream_t); \

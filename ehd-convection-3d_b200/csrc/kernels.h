@@ -219,6 +219,8 @@ template <typename R> cudaError_t launch_dft_cols(const PoissonArgs &a, int sign
 // modes per block of the shared-memory z solve, 0: the columns do not fit
 int zmeet_modes(int nz, size_t rsize);
 template <typename R> cudaError_t launch_zmeet(const PoissonArgs &a, cudaStream_t s);
+// sets its shared-memory attribute (before any stream capture; prepare_dft does)
+template <typename R> cudaError_t prepare_zmeet();
 
 // ---- diagnostics ---------------------------------------------------------
 

@@ -49,6 +49,11 @@ std::mutex g_mu;
 // the array may move)
 void *g_scratch_addr[kMaxDevices] = {};
 CUcontext g_scratch_ctx[kMaxDevices] = {};
+// the context in which the z solve's shared-memory attribute was set: its need
+// grows with NZ, so it is set by the first call outside a capture, whatever that
+// call's NZ, for a deeper one inside a capture
+CUcontext g_zmeet_ctx[kMaxDevices] = {};
+bool g_zmeet_set[kMaxDevices] = {};
 
 // The calling thread's current driver context, through the runtime's driver
 // entry point (the library links only the runtime).
@@ -192,6 +197,7 @@ extern "C" int ehd_poisson_noalloc(const ehd_params *p, const double *q, double 
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
         return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: no usable current device");
     unsigned char *base = nullptr;
+    cudaStream_t s = (cudaStream_t)stream;
     {
         // first call on this device (in this context): the device address of
         // the array
@@ -205,8 +211,15 @@ extern "C" int ehd_poisson_noalloc(const ehd_params *p, const double *q, double 
             g_scratch_ctx[dev] = ctx;
         }
         base = (unsigned char *)g_scratch_addr[dev];
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if ((!g_zmeet_set[dev] || g_zmeet_ctx[dev] != ctx) &&
+            cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) {
+            if (prepare_zmeet<double>() != cudaSuccess)
+                return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: kernel set-up failed");
+            g_zmeet_set[dev] = true;
+            g_zmeet_ctx[dev] = ctx;
+        }
     }
-    cudaStream_t s = (cudaStream_t)stream;
     PoissonArgs a{};
     a.nx = nx;
     a.ny = ny;
