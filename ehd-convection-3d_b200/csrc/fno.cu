@@ -806,8 +806,22 @@ Dims dims(const ehd_fno *f, int B) {
         if (e_ != cudaSuccess) return cuda_fail(#call, e_); \
     } while (0)
 
-// u: the caller's output array (any alignment), or nullptr: the output goes to
-// f->u and the hidden activations are kept for the backward pass
+// whether kernels on the device may store floats at p: aligned, and this
+// device's or managed memory
+bool stores_to(const float *p, int device) {
+    if ((uintptr_t)p % sizeof(float)) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == device);
+}
+
+// u: the caller's output array, or nullptr: the output goes to f->u and the
+// hidden activations are kept for the backward pass.  A u that a kernel may not
+// write is reached by a copy from f->u, which takes any alignment and any
+// device's memory, or refuses the pointer.
 int forward(ehd_fno *f, int B, const float *a, float *u) {
     const Dims d = dims(f, B);
     const size_t rows = (size_t)B * f->P;
@@ -830,7 +844,7 @@ int forward(ehd_fno *f, int B, const float *a, float *u) {
         FNO_CK(gemm(g, s));
     }
     const float *vL = f->z[f->L - 1];
-    if (u && project_usable((long long)rows, f->W, f->H, f->cout, vL)) {
+    if (u && project_usable((long long)rows, f->W, f->H, f->cout, vL) && stores_to(u, f->c.device)) {
         FNO_CK(project((long long)rows, f->W, f->H, f->cout, vL, pb + f->oQ1, f->param + f->oq1,
                        pb + f->oQ2, f->param + f->oq2, u, s));
         return EHD_OK;
