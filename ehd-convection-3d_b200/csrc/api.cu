@@ -616,7 +616,7 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
     }
     {
         // room for the plane sums of every launch shape ehd_set_tuning allows
-        c->pair = lbm_pair_usable(nx, c->sc.n, c->prec);
+        c->pair = lbm_pair_usable(nx, nz, c->sc.n, c->prec);
         int slots = c->rows_grid > 0 ? lbm_rows_slots_per_plane(nx, ny) : 0;
         if (c->pair) slots = std::max(slots, lbm_pair_slots(nx, ny));
         for (int bx = 16; bx <= 128; bx *= 2) slots = std::max(slots, lbm_blocks_per_plane(nx, ny, bx));

@@ -24,7 +24,7 @@ struct LbmArgs {
 
 // ---- two nodes per thread, FP32 and FP16 flow populations (csrc/lbm_pair.cu) ----
 // whether it serves a grid of n nodes (prec: ehd_precision); psum slots per plane
-bool lbm_pair_usable(int nx, long long n, int prec);
+bool lbm_pair_usable(int nx, int nz, long long n, int prec);
 int lbm_pair_slots(int nx, int ny);
 cudaError_t launch_lbm_pair(int prec, const LbmArgs &a, const StepConst &c, bool macros,
                             cudaStream_t s);

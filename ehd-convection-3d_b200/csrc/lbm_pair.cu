@@ -362,9 +362,10 @@ int lbm_pair_slots(int nx, int ny) {
 }
 
 // FP32, or FP16 f with FP16 or FP32 g; rows of whole pairs, 32-bit byte
-// offsets of the 4-byte arrays
-bool lbm_pair_usable(int nx, long long n, int prec) {
-    return (prec == 1 || prec == 2 || prec == 4) && nx % 2 == 0 && n < (1LL << 30);
+// offsets of the 4-byte arrays, and NZ + 1 blocks along y where plane 0 goes
+// with the pairs
+bool lbm_pair_usable(int nx, int nz, long long n, int prec) {
+    return (prec == 1 || prec == 2 || prec == 4) && nx % 2 == 0 && nz < 65535 && n < (1LL << 30);
 }
 
 // Up to so many blocks of pairs plane 0 goes with them: 64 x 64 x 33 in FP16
