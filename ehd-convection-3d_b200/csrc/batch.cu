@@ -489,13 +489,15 @@ int ehd_batch_run_to_saturation(ehd_batch *b, int sample_every, double tol, int 
     return EHD_OK;
 }
 
-namespace {
+namespace ehd {
 
-// average time of one batch step over `steps` steps of every instance (after
-// one untimed step, which also captures a new graph if the shapes changed)
-// The time of one batch step: the best of three runs of `steps` steps after a
-// warm-up step (the shortest run is the one least disturbed).
-int time_batch(ehd_batch *b, const std::vector<char> &act, int steps, float *ms) {
+// The time of one batch step of all instances: the best of three runs of `steps`
+// steps (the shortest run is the one least disturbed) after a warm-up step, which
+// also captures a new graph if the shapes changed.  The events stand on the batch stream behind
+// every instance's: columns step on their own streams, which it does not wait for
+// otherwise.
+int batch_step_time(ehd_batch *b, int steps, float *ms) {
+    const std::vector<char> act(b->inst.size(), 1);
     int r = batch_step(b, act, 1);
     if (r != EHD_OK) return r;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -504,8 +506,10 @@ int time_batch(ehd_batch *b, const std::vector<char> &act, int steps, float *ms)
     float best = 0.f;
     cudaError_t e = cudaSuccess;
     for (int rep = 0; rep < 3 && r == EHD_OK && e == cudaSuccess; ++rep) {
+        if ((r = order(b, act, true)) != EHD_OK) break;
         cudaEventRecord(e0, b->stream);
         r = batch_step(b, act, steps);
+        if (r == EHD_OK) r = order(b, act, true);
         cudaEventRecord(e1, b->stream);
         e = cudaEventSynchronize(e1);
         float t = 0.f;
@@ -520,7 +524,7 @@ int time_batch(ehd_batch *b, const std::vector<char> &act, int steps, float *ms)
     return EHD_OK;
 }
 
-}  // namespace
+}  // namespace ehd
 
 // The autotuner times the whole batch, not instances alone: the instances'
 // kernels share the GPU, so the shape that is fastest for a grid alone is not
@@ -549,7 +553,7 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
     for (size_t i = 0; r == EHD_OK && i < n; ++i) r = ehd_initialize(s->inst[i]);
     if (r == EHD_OK) r = batch_step(s, all, 1);
     float best_ms = 0.f;
-    if (r == EHD_OK) r = time_batch(s, all, trial_steps, &best_ms);
+    if (r == EHD_OK) r = batch_step_time(s, trial_steps, &best_ms);
     std::vector<ehd_tuning> choice, start;
     for (auto &g : groups) {
         ehd_tuning t{};
@@ -571,7 +575,7 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
                 return EHD_OK;
             }
             float ms = 0.f;
-            int rr = time_batch(s, all, trial_steps, &ms);
+            int rr = batch_step_time(s, trial_steps, &ms);
             if (rr != EHD_OK) return rr;
             if (ms < 0.99f * best_ms) {
                 best_ms = ms;
@@ -628,8 +632,8 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
             return true;
         };
         float chosen_ms = 0.f, start_ms = 0.f;
-        if (apply_all(choice)) r = time_batch(s, all, trial_steps, &chosen_ms);
-        if (r == EHD_OK && apply_all(start)) r = time_batch(s, all, trial_steps, &start_ms);
+        if (apply_all(choice)) r = batch_step_time(s, trial_steps, &chosen_ms);
+        if (r == EHD_OK && apply_all(start)) r = batch_step_time(s, trial_steps, &start_ms);
         if (r == EHD_OK && start_ms > 0.f && start_ms <= chosen_ms) choice = start;
     }
     ehd_batch_destroy(s);
