@@ -455,6 +455,23 @@ int ctx_parity(const ehd_ctx *c) { return c->cur; }
 int ctx_capture_steps(ehd_ctx *c, int steps, bool macros) { return capture_steps(c, steps, macros); }
 unsigned ctx_generation(const ehd_ctx *c) { return c->generation; }
 void ctx_tuning(const ehd_ctx *c, ehd_tuning *t) { *t = c->tune; }
+ehd_tuning ctx_effective(const ehd_ctx *c, ehd_tuning t, bool grouped) {
+    const bool column = column_usable(c->p.nx, c->p.ny, c->p.nz);
+    if (column && t.lbm_kernel == 0) return ehd_tuning{};  // one kernel for the whole step
+    // the kernel that lbm_kernel = 0 stands for, as in lbm() and ctx_step_args()
+    const bool rows = c->rows_grid > 0 && (grouped || c->prec == EHD_PREC_FP64);
+    const bool own = rows || (c->pair && !grouped);
+    if (own && t.lbm_kernel == 0) t.node_block_x = 0;
+    if (!own && !column) t.lbm_kernel = 0;
+    // the Poisson solve, as in launch_poisson() and zsolve()
+    const PoissonArgs &a = c->pa;
+    const bool split = a.cps && t.poisson_path == 0;
+    if (!a.cps) t.poisson_path = 0;
+    if (split || !a.cpt || (!a.twz && zmeet_modes(c->p.nz, c->rsize) == 0)) t.z_solve = 0;
+    if (split || a.tabx || poisson_fast_size(c->p.nx)) t.fft_rows = 0;
+    if (split || a.taby || poisson_fast_size(c->p.ny)) t.fft_cols = 0;
+    return t;
+}
 int ctx_step_args(ehd_ctx *c, bool macros, LbmArgs *la, StepConst *sc, ReduceDesc *rd,
                   PoissonArgs *pa) {
     (void)macros;

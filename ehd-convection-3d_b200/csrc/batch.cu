@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <cstdint>
 #include <map>
 #include <string>
@@ -569,7 +570,18 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
                 if (ehd_set_tuning(s->inst[i], &t) != EHD_OK) return false;
             return true;
         };
+        // a trial of t, if it launches anything that was not timed yet
+        std::vector<ehd_tuning> timed;
+        auto is_new = [&](const ehd_tuning &t) {
+            const ehd_tuning e = ctx_effective(s->inst[g.second.front()], t, s->mode == 0);
+            for (const ehd_tuning &o : timed)
+                if (std::memcmp(&e, &o, sizeof e) == 0) return false;
+            timed.push_back(e);
+            return true;
+        };
+        (void)is_new(best);
         auto trial = [&](ehd_tuning t) -> int {
+            if (!is_new(t)) return EHD_OK;
             if (!apply(t)) {  // shape not allowed for this grid
                 apply(best);
                 return EHD_OK;
@@ -585,37 +597,34 @@ int ehd_batch_autotune(ehd_batch *b, int trial_steps) {
             }
             return EHD_OK;
         };
-        const ehd_params &p = ps[g.second.front()];
         for (int kern = 0; r == EHD_OK && kern <= 1; ++kern)
             for (int bx = 16; r == EHD_OK && bx <= 128; bx *= 2) {
                 ehd_tuning t = best;
                 t.lbm_kernel = kern;
                 t.node_block_x = bx;
-                if (t.lbm_kernel != best.lbm_kernel || t.node_block_x != best.node_block_x) r = trial(t);
+                r = trial(t);
             }
         if (r == EHD_OK) {  // the split-y or the five-kernel Poisson solve
             ehd_tuning t = best;
             t.poisson_path = 1 - best.poisson_path;
             r = trial(t);
         }
-        if (r == EHD_OK && !poisson_fast_size(2 * (p.nz - 1))) {  // which Thomas solve
+        if (r == EHD_OK) {  // the FP64 sweep or the faster z solve
             ehd_tuning t = best;
             t.z_solve = 1 - best.z_solve;
             r = trial(t);
         }
         // run-time radix passes
-        if (!poisson_fast_size(p.nx))
-            for (int rows = 1; r == EHD_OK && rows <= 32; rows *= 2) {
-                ehd_tuning t = best;
-                t.fft_rows = rows;
-                if (rows != best.fft_rows) r = trial(t);
-            }
-        if (!poisson_fast_size(p.ny))
-            for (int cols = 1; r == EHD_OK && cols <= 32; cols *= 2) {
-                ehd_tuning t = best;
-                t.fft_cols = cols;
-                if (cols != best.fft_cols) r = trial(t);
-            }
+        for (int rows = 1; r == EHD_OK && rows <= 32; rows *= 2) {
+            ehd_tuning t = best;
+            t.fft_rows = rows;
+            r = trial(t);
+        }
+        for (int cols = 1; r == EHD_OK && cols <= 32; cols *= 2) {
+            ehd_tuning t = best;
+            t.fft_cols = cols;
+            r = trial(t);
+        }
         choice.push_back(best);
     }
     // coordinate descent over the grids can end worse than where it began

@@ -272,6 +272,9 @@ void ctx_commit_steps(::ehd_ctx *c, int steps);
 unsigned ctx_generation(const ::ehd_ctx *c);
 // the context's launch shapes
 void ctx_tuning(const ::ehd_ctx *c, ::ehd_tuning *t);
+// t with 0 in the fields that change no launch of the context's steady steps
+// (grouped: in a batch with grouped launches)
+::ehd_tuning ctx_effective(const ::ehd_ctx *c, ::ehd_tuning t, bool grouped);
 // the arguments of one steady step at the context's present buffer parity,
 // with the LBM half on the per-node kernel (what a launch over a group of
 // instances runs); nothing is launched

@@ -1,4 +1,4 @@
-"""What the batch autotuner measures (csrc/batch.cu, batch_step_time)."""
+"""What the batch autotuner measures (csrc/batch.cu, batch_step_time) and what it tries."""
 import ctypes
 import time
 
@@ -37,3 +37,34 @@ def test_columns_are_timed():
         ms = ctypes.c_float()
         assert step_time(b.h, steps, ctypes.byref(ms)) == 0
         assert 0.5 < 1e-3 * ms.value * steps / min(wall) < 1.5, (ms.value * steps, wall)
+
+
+# (grid, storage, grouped launches, fields that reach no launch while lbm_kernel and
+# poisson_path stay 0): a column; folded axes, on pairs, on the per-node kernel (odd
+# NX) and, FP64, on rows; the split-y solve; run-time passes (BF16 storage), where all
+# but lbm_kernel count
+IDLE = [((1, 1, 33), "fp32", False, ("node_block_x", "fft_rows", "fft_cols", "poisson_path", "z_solve")),
+        ((24, 22, 9), "fp32", False, ("node_block_x", "fft_rows", "fft_cols", "poisson_path")),
+        ((23, 22, 9), "fp32", False, ("lbm_kernel", "fft_rows", "fft_cols", "poisson_path")),
+        ((44, 22, 9), "fp64", False, ("node_block_x", "fft_rows", "fft_cols", "poisson_path")),
+        ((64, 64, 33), "fp32", False, ("node_block_x", "fft_rows", "fft_cols", "z_solve")),
+        ((64, 64, 33), "fp16", True, ("lbm_kernel", "fft_rows", "fft_cols", "z_solve")),
+        ((24, 22, 9), "bf16", False, ("lbm_kernel", "poisson_path"))]
+
+
+@pytest.mark.parametrize("shape,prec,grouped,idle", IDLE)
+def test_fields_without_effect_are_not_tried(shape, prec, grouped, idle):
+    """Trials of fields that change no launch time the same launches again, and noise
+    chooses among them: three short autotunes leave such fields as they were, as long
+    as the kernel and the path that make them idle are kept."""
+    with ehd.Batch([params(*shape)] * 2, prec) as b:
+        b.set_mode(0 if grouped else 1)
+        start = b[0].get_tuning()
+        for _ in range(3):
+            b.autotune(trial_steps=1)
+            t = b[0].get_tuning()
+            if t["lbm_kernel"] == 0 and t["poisson_path"] == 0:
+                for k in idle:
+                    assert t[k] == start[k], (k, t, start)
+            if "lbm_kernel" in idle:
+                assert t["lbm_kernel"] == 0
