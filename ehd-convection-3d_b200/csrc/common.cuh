@@ -153,9 +153,12 @@ inline cudaError_t set_smem(K kern, size_t bytes, cudaStream_t s) {
 __device__ __forceinline__ void step_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-template <typename... P, typename... A>
+// The arguments convert to the kernel's parameters implicitly, as in a <<<>>>
+// launch: a pointer of another type does not compile.
+template <typename T> struct NotDeduced { using type = T; };
+template <typename... P>
 inline cudaError_t step_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                               cudaStream_t s, A &&...args) {
+                               cudaStream_t s, const typename NotDeduced<P>::type &...args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -166,7 +169,7 @@ inline cudaError_t step_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+    return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 template <typename T> struct Store;
