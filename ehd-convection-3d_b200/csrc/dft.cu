@@ -201,7 +201,7 @@ template <typename R, int TN, bool EVEN>
 __global__ void __launch_bounds__(kThreads, min_blocks<R>())
 dft_rows_fwd(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec,
              double *__restrict__ rowsum, const typename Cplx<R>::T *__restrict__ tab, int tp,
-             const double *__restrict__ qmean, int nx, int ny, int rows, int nxh, int pitch,
+             const double *__restrict__ qmean, int nx, int ny, int rows, int pitch,
              double eps, const PoissonPtrs *__restrict__ grp) {
     step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
@@ -323,7 +323,7 @@ template <typename R, int TN, bool EVEN>
 __global__ void __launch_bounds__(kThreads, min_blocks<R>())
 dft_rows_inv(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phip,
              const typename Cplx<R>::T *__restrict__ tab, int tp, int nx, int ny, int rows,
-             int nxh, int pitch, const PoissonPtrs *__restrict__ grp) {
+             int pitch, const PoissonPtrs *__restrict__ grp) {
     step_enter();
     if (grp) {  // one instance of a group launch per blockIdx.z
         const PoissonPtrs &gp = grp[blockIdx.z];
@@ -915,9 +915,9 @@ cudaError_t launch_dft_rows_fwd(const PoissonArgs &a, cudaStream_t s) {
         auto kern = dft_rows_fwd<R, TN, decltype(even)::value>;
         cudaError_t e = set_smem(kern, rows_smem<R, TN>(), s);
         if (e != cudaSuccess) return e;
-        step_launch(kern, grid, kThreads, rows_smem<R, TN>(), s, 
-            (const R *)a.q, (R2 *)a.spec, a.rowsum, (const R2 *)a.tabx, tp, a.qmean, a.nx, a.ny,
-            rows, a.nxh, a.pitch, a.eps, a.grp);
+        step_launch(kern, grid, kThreads, rows_smem<R, TN>(), s, (const R *)a.q, (R2 *)a.spec,
+                    a.rowsum, (const R2 *)a.tabx, tp, a.qmean, a.nx, a.ny, rows, a.pitch, a.eps,
+                    a.grp);
         return cudaGetLastError();
     });
 }
@@ -931,9 +931,8 @@ cudaError_t launch_dft_rows_inv(const PoissonArgs &a, cudaStream_t s) {
         auto kern = dft_rows_inv<R, TN, decltype(even)::value>;
         cudaError_t e = set_smem(kern, rows_smem<R, TN>(), s);
         if (e != cudaSuccess) return e;
-        step_launch(kern, grid, kThreads, rows_smem<R, TN>(), s, 
-            (const R2 *)a.spec, (R *)a.phip, (const R2 *)a.tabx, tp, a.nx, a.ny, rows, a.nxh,
-            a.pitch, a.grp);
+        step_launch(kern, grid, kThreads, rows_smem<R, TN>(), s, (const R2 *)a.spec, (R *)a.phip,
+                    (const R2 *)a.tabx, tp, a.nx, a.ny, rows, a.pitch, a.grp);
         return cudaGetLastError();
     });
 }
@@ -948,9 +947,8 @@ cudaError_t launch_dft_cols(const PoissonArgs &a, int sign, cudaStream_t s) {
                              : dft_cols<R, 1, TN, decltype(even)::value>;
         cudaError_t e = set_smem(kern, cols_smem<R, TN>(), s);
         if (e != cudaSuccess) return e;
-        step_launch(kern, grid, kThreads, cols_smem<R, TN>(), s, 
-            (const R2 *)(sign < 0 ? a.spec : a.spec2), (R2 *)(sign < 0 ? a.spec2 : a.spec),
-            (const R2 *)a.taby, tp, a.ny, a.nxh, a.pitch, mtiles, a.rowsum, a.planesum, a.grp);
+        step_launch(kern, grid, kThreads, cols_smem<R, TN>(), s,
+                    (const R2 *)(sign < 0 ? a.spec : a.spec2), (R2 *)(sign < 0 ? a.spec2 : a.spec), (const R2 *)a.taby, tp, a.ny, a.nxh, a.pitch, mtiles, a.rowsum, a.planesum, a.grp);
         return cudaGetLastError();
     });
 }
@@ -972,10 +970,10 @@ cudaError_t launch_zmeet(const PoissonArgs &a, cudaStream_t s) {
     const size_t sm = cols > mean ? cols : mean;
     cudaError_t e = set_smem(poisson_zmeet<R>, sm, s);
     if (e != cudaSuccess) return e;
-    step_launch(poisson_zmeet<R>, dim3((modes + mb - 1) / mb + 1, 1, a.ngrp), 128, sm, s, 
-        (R2 *)a.spec, a.cpt, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny,
-        a.nz, a.nxh, a.pitch, mb, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx, 2.0 * M_PI / a.ly,
-        a.grp);
+    step_launch(poisson_zmeet<R>, dim3((modes + mb - 1) / mb + 1, 1, a.ngrp), 128, sm, s,
+                (R2 *)a.spec, a.cpt, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz,
+                a.nxh, a.pitch, mb, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx, 2.0 * M_PI / a.ly,
+                a.grp);
     return cudaGetLastError();
 }
 

@@ -374,7 +374,7 @@ bool aligned16(const void *a) { return ((uintptr_t)a & 15) == 0; }
 void gelu_back(float *d, const float *z, size_t n, cudaStream_t s) {
     if (n % 4 == 0 && aligned16(d) && aligned16(z))
         step_launch(gelu_back4_kernel, grid_for(n / 8), 256, 0, s, reinterpret_cast<float4 *>(d),
-                                                         reinterpret_cast<const float4 *>(z), n / 4);
+                    reinterpret_cast<const float4 *>(z), n / 4);
     else
         step_launch(gelu_back_kernel, grid_for(n), 256, 0, s, d, z, n);
 }
@@ -507,8 +507,8 @@ cudaError_t refresh(ehd_fno *f) {
     for (int l = 0; l <= f->L; ++l) {
         const size_t to = l < f->L ? f->lo[l].Rre : f->nparam;
         if (to > from)
-            step_launch(cast_bf16_kernel, grid_for(to - from), 256, 0, f->stream, f->param + from,
-                                                                         f->pbf + from, to - from);
+            step_launch(cast_bf16_kernel, grid_for(to - from), 256, 0,
+                        f->stream, f->param + from, f->pbf + from, to - from);
         if (l < f->L) from = f->lo[l].Rim + spec;
     }
     return cudaGetLastError();
@@ -791,8 +791,8 @@ cudaError_t mix(const ehd_fno *f, int l, const float *in, float *out, int B, boo
 cudaError_t mix_wgrad(const ehd_fno *f, int l, const float *dout, const float *x, float *g, int B) {
     const int nw = mix_warps(f->W, (size_t)16 * f->W);
     const unsigned blocks = (unsigned)std::min<size_t>((f->modes + nw - 1) / nw, 148 * 16);
-    step_launch(mix_wgrad_kernel, blocks, 32 * nw, (size_t)nw * 16 * f->W * sizeof(float), f->stream, 
-        dout, x, g + f->lo[l].Rre, g + f->lo[l].Rim, f->modes, f->W, B);
+    step_launch(mix_wgrad_kernel, blocks, 32 * nw,
+                (size_t)nw * 16 * f->W * sizeof(float), f->stream, dout, x, g + f->lo[l].Rre, g + f->lo[l].Rim, f->modes, f->W, B);
     return cudaGetLastError();
 }
 
@@ -1116,11 +1116,11 @@ int ehd_fno_adam_step(ehd_fno *f, float lr, float b1, float b2, float eps) {
     f->adam_t += 1;
     const float c1 = 1.f - std::pow(b1, (float)f->adam_t), c2 = 1.f - std::pow(b2, (float)f->adam_t);
     if (aligned16(f->param) && aligned16(f->grad) && aligned16(f->adam_m) && aligned16(f->adam_v))
-        step_launch(adam4_kernel, grid_for(f->nparam / 4 + 1), 256, 0, f->stream, 
-            f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
+        step_launch(adam4_kernel,
+                    grid_for(f->nparam / 4 + 1), 256, 0, f->stream, f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
     else
-        step_launch(adam_kernel, grid_for(f->nparam), 256, 0, f->stream, 
-            f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
+        step_launch(adam_kernel,
+                    grid_for(f->nparam), 256, 0, f->stream, f->param, f->grad, f->adam_m, f->adam_v, f->nparam, lr, b1, b2, eps, c1, c2);
     FNO_CK(cudaGetLastError());
     FNO_CK(refresh(f));
     return EHD_OK;

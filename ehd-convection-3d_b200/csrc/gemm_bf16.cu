@@ -1213,7 +1213,7 @@ cudaError_t weight_bias_grad(long long rows, int M, int N, const float *X, int l
         const long long chunks = (rows + 15) / 16;
         const long long blocks = std::min((chunks + 7) / 8, (long long)nsm * std::max(occ, 1));
         step_launch(k, (unsigned)blocks, 256, 0, s, X, ldx, M, D + n0, ldd, nn, rows, G + n0, ldg,
-                                          gb ? gb + n0 : nullptr);
+                    gb ? gb + n0 : nullptr);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -177,8 +177,9 @@ lbm_pair_kernel(const Args a, const KConst<float> c) {
     // node of a plane (FP32, 64 x 64 x 33, 100 steps, 24 starts: distance of u and
     // phi from the 64-bit run 1.012 and 1.006 times the per-node kernel's, 1.000
     // and 1.001 so).  256 x 256 x 129 in FP32 643 us a step, 640 with the rounded
-    // products; 122 x 122 x 101 167 and 161.  16-bit f direction by direction of e_z, which leaves the kernel
-    // registers for more loads: FP16 499 us, in the order of d 508.
+    // products; 122 x 122 x 101 167 and 161.  16-bit f by e_z, which leaves the
+    // kernel registers for more loads: 256 x 256 x 129 in FP16 499 us, in the order
+    // of d 508.
     auto shift = [&](int d) {
         const float2 w = dup(c.w[cls_of(d)]);
         f[d] = fma2(w, dup(ez_of(d) > 0 ? zr[2] : (ez_of(d) < 0 ? zr[4] : zr[3])), f[d]);

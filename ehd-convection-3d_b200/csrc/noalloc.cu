@@ -270,8 +270,8 @@ extern "C" int ehd_poisson_noalloc(const ehd_params *p, const double *q, double 
         return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: the table kernel failed to launch");
     if (launch_poisson<double>(a, s) != cudaSuccess)
         return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: Poisson kernels failed to launch");
-    if (step_launch(fields_kernel, dim3((nx * ny + 255) / 256, nz), 256, 0, s, phip, a.phi00, phi, ex, ey, ez, nx, ny, nz,
-                    0.5 / p->dx, 0.5 / p->dy, 0.5 / p->dz) != cudaSuccess)
+    if (step_launch(fields_kernel, dim3((nx * ny + 255) / 256, nz), 256, 0, s, phip, a.phi00, phi,
+                    ex, ey, ez, nx, ny, nz, 0.5 / p->dx, 0.5 / p->dy, 0.5 / p->dz) != cudaSuccess)
         return set_error(EHD_ERR_CUDA, "ehd_poisson_noalloc: the field kernel failed to launch");
     return EHD_OK;
 }

@@ -1587,9 +1587,8 @@ static cudaError_t rows_fwd_fast(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_rows_fwd_fast<R, N>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * TB - 1) / (2 * TB), a.nz - 2, a.ngrp);
-    step_launch(poisson_rows_fwd_fast<R, N>, grid, 256, sm, s, (const R *)a.q, (R2 *)a.spec, a.rowsum,
-                                                       (const R2 *)a.twx, a.qmean,
-                                                       a.ny, a.nxh, a.pitch, a.eps, a.grp);
+    step_launch(poisson_rows_fwd_fast<R, N>, grid, 256, sm, s, (const R *)a.q, (R2 *)a.spec,
+                a.rowsum, (const R2 *)a.twx, a.qmean, a.ny, a.nxh, a.pitch, a.eps, a.grp);
     return cudaGetLastError();
 }
 template <typename R, int N>
@@ -1601,7 +1600,7 @@ static cudaError_t rows_inv_fast(const PoissonArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * TB - 1) / (2 * TB), a.nz - 2, a.ngrp);
     step_launch(poisson_rows_inv_fast<R, N>, grid, 256, sm, s, (const R2 *)a.spec, (R *)a.phip,
-                                                       (const R2 *)a.twx, a.ny, a.nxh, a.pitch, a.grp);
+                (const R2 *)a.twx, a.ny, a.nxh, a.pitch, a.grp);
     return cudaGetLastError();
 }
 template <typename R, int N, int S>
@@ -1612,8 +1611,8 @@ static cudaError_t cols_fast(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_cols_fast<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nxh + TB - 1) / TB, a.nz - 2, a.ngrp);
-    step_launch(poisson_cols_fast<R, N, S>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy, a.nxh,
-                                                      a.pitch, a.rowsum, a.planesum, a.grp);
+    step_launch(poisson_cols_fast<R, N, S>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy,
+                a.nxh, a.pitch, a.rowsum, a.planesum, a.grp);
     return cudaGetLastError();
 }
 
@@ -1637,8 +1636,7 @@ static cudaError_t rows_fwd(const PoissonArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * rows - 1) / (2 * rows), a.nz - 2, a.ngrp);
     step_launch(poisson_rows_fwd<R>, grid, 256, sm, s, (const R *)a.q, (R2 *)a.spec, a.rowsum,
-                                               (const R2 *)a.twx, a.qmean, a.px,
-                                               a.nx, a.ny, a.nxh, a.pitch, rows, a.eps, a.grp);
+                (const R2 *)a.twx, a.qmean, a.px, a.nx, a.ny, a.nxh, a.pitch, rows, a.eps, a.grp);
     return cudaGetLastError();
 }
 template <typename R>
@@ -1661,8 +1659,7 @@ static cudaError_t rows_inv(const PoissonArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     dim3 grid((a.ny + 2 * rows - 1) / (2 * rows), a.nz - 2, a.ngrp);
     step_launch(poisson_rows_inv<R>, grid, 256, sm, s, (const R2 *)a.spec, (R *)a.phip,
-                                               (const R2 *)a.twx, a.px, a.nx, a.ny, a.nxh,
-                                               a.pitch, rows, a.grp);
+                (const R2 *)a.twx, a.px, a.nx, a.ny, a.nxh, a.pitch, rows, a.grp);
     return cudaGetLastError();
 }
 template <typename R, int S>
@@ -1684,9 +1681,9 @@ static cudaError_t cols(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_cols<R>, sm, s);
     if (e != cudaSuccess) return e;
     dim3 grid((a.nxh + cc - 1) / cc, a.nz - 2, a.ngrp);
-    step_launch(poisson_cols<R>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy, a.py, a.ny, a.nxh,
-                                           a.pitch, cc, (R)S, S < 0 ? a.rowsum : nullptr,
-                                           S < 0 ? a.planesum : nullptr, a.grp);
+    step_launch(poisson_cols<R>, grid, 256, sm, s, (R2 *)a.spec, (const R2 *)a.twy, a.py, a.ny,
+                a.nxh, a.pitch, cc, (R)S,
+                S < 0 ? a.rowsum : nullptr, S < 0 ? a.planesum : nullptr, a.grp);
     return cudaGetLastError();
 }
 
@@ -1699,9 +1696,10 @@ static cudaError_t zdst(const PoissonArgs &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int modes = a.nxh * a.ny;
     const R2 *tw = (const R2 *)a.twz;
-    step_launch(poisson_zdst<R, L>, dim3((modes + TB - 1) / TB, 1, a.ngrp), 256, sm, s, 
-        (R2 *)a.spec, tw, (const R *)(tw + L), a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny,
-        a.nxh, a.pitch, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx, 2.0 * M_PI / a.ly, a.grp);
+    step_launch(poisson_zdst<R, L>, dim3((modes + TB - 1) / TB, 1, a.ngrp), 256, sm, s,
+                (R2 *)a.spec, tw, (const R *)(tw + L), a.planesum, a.qmean, a.phi00, a.ez00, a.nx,
+                a.ny, a.nxh, a.pitch, a.dz, a.eps, a.voltage, 2.0 * M_PI / a.lx,
+                2.0 * M_PI / a.ly, a.grp);
     return cudaGetLastError();
 }
 
@@ -1720,9 +1718,9 @@ static cudaError_t split_rows_fwd(const PoissonArgs &a, cudaStream_t s) {
     const size_t sm = sizeof(R2) * ((size_t)N + (size_t)TB * tstride<N>());
     cudaError_t e = set_smem(poisson_rows_fwd_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
-    step_launch(poisson_rows_fwd_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s, 
-        (const R *)a.q, (R2 *)a.spec, a.rowsum, (const R2 *)a.twx, (const R2 *)a.twy, a.qmean,
-        a.nz - 2, a.nxh, a.eps, a.grp);
+    step_launch(poisson_rows_fwd_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s,
+                (const R *)a.q, (R2 *)a.spec, a.rowsum, (const R2 *)a.twx, (const R2 *)a.twy,
+                a.qmean, a.nz - 2, a.nxh, a.eps, a.grp);
     return cudaGetLastError();
 }
 template <typename R, int N, int S>
@@ -1732,8 +1730,9 @@ static cudaError_t split_rows_inv(const PoissonArgs &a, cudaStream_t s) {
     constexpr size_t sm = rows_inv_split_smem<R, N, S>();
     cudaError_t e = set_smem(poisson_rows_inv_split<R, N, S>, sm, s);
     if (e != cudaSuccess) return e;
-    step_launch(poisson_rows_inv_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s, 
-        (const R2 *)a.spec, (R *)a.phip, (const R2 *)a.twx, (const R2 *)a.twy, a.nz - 2, a.nxh, a.grp);
+    step_launch(poisson_rows_inv_split<R, N, S>, dim3(64 / NB, a.nz - 2, a.ngrp), 256, sm, s,
+                (const R2 *)a.spec, (R *)a.phip, (const R2 *)a.twx, (const R2 *)a.twy, a.nz - 2,
+                a.nxh, a.grp);
     return cudaGetLastError();
 }
 template <typename R, int L, int S>
@@ -1743,9 +1742,9 @@ static cudaError_t split_slab(const PoissonArgs &a, cudaStream_t s) {
     cudaError_t e = set_smem(poisson_slab<R, L, S>, sm, s);
     if (e != cudaSuccess) return e;
     // one block more than kx columns: block x = 0 solves the mean mode
-    step_launch(poisson_slab<R, L, S>, dim3(a.nxh + 1, S, a.ngrp), 256, sm, s, 
-        (R2 *)a.spec, (const R2 *)a.twy, (const R *)a.cps, a.rowsum, a.planesum, a.qmean,
-        a.phi00, a.ez00, a.nx, a.nxh, a.dz, a.eps, a.voltage, a.grp);
+    step_launch(poisson_slab<R, L, S>, dim3(a.nxh + 1, S, a.ngrp), 256, sm, s, (R2 *)a.spec,
+                (const R2 *)a.twy, (const R *)a.cps, a.rowsum, a.planesum, a.qmean, a.phi00,
+                a.ez00, a.nx, a.nxh, a.dz, a.eps, a.voltage, a.grp);
     return cudaGetLastError();
 }
 
@@ -1925,9 +1924,9 @@ static cudaError_t zsolve(const PoissonArgs &a0, cudaStream_t s) {
         return cudaGetLastError();
     }
     if (!a.thomas && zmeet_modes(a.nz, sizeof(R)) > 0) return launch_zmeet<R>(a, s);
-    step_launch(poisson_zsolve<R>, dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s, 
-        (R2 *)a.spec, a.cpt, a.dpw, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz,
-        a.nxh, a.pitch, a.dz, a.eps, a.voltage, a.grp);
+    step_launch(poisson_zsolve<R>, dim3((modes + 127) / 128, 1, a.ngrp), 128, 0, s, (R2 *)a.spec,
+                a.cpt, a.dpw, a.planesum, a.qmean, a.phi00, a.ez00, a.nx, a.ny, a.nz, a.nxh,
+                a.pitch, a.dz, a.eps, a.voltage, a.grp);
     return cudaGetLastError();
 }
 
