@@ -106,6 +106,7 @@ struct ehd_ctx {
     float2 *psum = nullptr;
     int psum_blocks = 0;   // psum slots per plane of the per-node kernel
     int rows_grid = 0;     // CTAs of the bulk-copy row kernel, 0: not available
+    int rows_group = 0;    // and of a group of instances on this grid
     bool pair = false;     // two nodes per thread (lbm_pair.cu) available
     ehd_tuning tune{};     // launch shapes (ehd_set_tuning)
     unsigned generation = 0;  // bumped by ehd_set_tuning
@@ -497,7 +498,7 @@ int ctx_step_args(ehd_ctx *c, bool macros, LbmArgs *la, StepConst *sc, ReduceDes
     // the steady-state step's kernel, as in lbm(): the row kernel where it is
     // available and chosen, else the per-node kernel
     const bool rows = c->rows_grid > 0 && c->tune.lbm_kernel == 0;
-    a.rows_grid = rows ? c->rows_grid : 0;
+    a.rows_grid = rows ? c->rows_group : 0;
     a.node_bx = c->tune.node_block_x;
     *la = a;
     *sc = c->sc;
@@ -619,11 +620,11 @@ int ehd_create(const ehd_params *params, const ehd_config *config, ehd_ctx **out
         // the bulk-copy row kernel for steady-state steps, where it applies
         cudaError_t e = cudaSuccess;
         switch (c->prec) {
-            case EHD_PREC_FP64: e = prepare_lbm_rows<double, double>(nx, ny, nz, &c->rows_grid); break;
-            case EHD_PREC_FP32: e = prepare_lbm_rows<float, float>(nx, ny, nz, &c->rows_grid); break;
-            case EHD_PREC_FP16: e = prepare_lbm_rows<__half, float>(nx, ny, nz, &c->rows_grid); break;
-            case EHD_PREC_MIXED: e = prepare_lbm_rows<Mix16, float>(nx, ny, nz, &c->rows_grid); break;
-            default: e = prepare_lbm_rows<__nv_bfloat16, float>(nx, ny, nz, &c->rows_grid); break;
+            case EHD_PREC_FP64: e = prepare_lbm_rows<double, double>(nx, ny, nz, &c->rows_grid, &c->rows_group); break;
+            case EHD_PREC_FP32: e = prepare_lbm_rows<float, float>(nx, ny, nz, &c->rows_grid, &c->rows_group); break;
+            case EHD_PREC_FP16: e = prepare_lbm_rows<__half, float>(nx, ny, nz, &c->rows_grid, &c->rows_group); break;
+            case EHD_PREC_MIXED: e = prepare_lbm_rows<Mix16, float>(nx, ny, nz, &c->rows_grid, &c->rows_group); break;
+            default: e = prepare_lbm_rows<__nv_bfloat16, float>(nx, ny, nz, &c->rows_grid, &c->rows_group); break;
         }
         if (e != cudaSuccess) return bail(fail(EHD_ERR_CUDA, "row kernel set-up: %s", cudaGetErrorString(e)));
     }

@@ -103,9 +103,10 @@ int lbm_default_block_x(int nx, bool bf16);
 // whether the bulk-copy row kernel serves this grid and storage type
 bool lbm_rows_usable(int nx, size_t fsize, size_t gsize);
 // sets the row kernel's shared-memory attribute (before any stream capture)
-// and returns its persistent grid size in *grid, 0 when it does not apply
+// and returns its persistent grid size in *grid (the CTAs that walk rows) and that
+// of a group in *group, 0 when it does not apply
 template <typename T, typename R>
-cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid);
+cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid, int *group);
 // psum slots per plane: per-node kernel / row kernel
 int lbm_rows_slots_per_plane(int nx, int ny);
 

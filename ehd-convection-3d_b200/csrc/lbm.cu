@@ -62,7 +62,7 @@ lbm_step_kernel(const StepArgs<T, R> a, const KConst<R> c, int local_pops, int e
 // of the stage (shared counter); the warp that counts last refills the stage
 // with the row two iterations ahead while the others compute.  The injector
 // plane z = 0 (own-node g and z = 1 populations) is left to CTAs of its own
-// (rows_cta).  A wait that does not complete within
+// (rows_cta), in a group to a launch of its own.  A wait that does not complete within
 // kWaitLimit polls sets *err, waits (bounded) for the copies that may still
 // be landing, and ends the warp.
 //
@@ -247,7 +247,7 @@ lbm_rows_group_kernel(const LbmGroupDesc<T, R> *__restrict__ desc) {
     __shared__ LbmGroupDesc<T, R> sd;
     load_group_desc(sd, desc, (int)blockIdx.y);
     __syncthreads();
-    rows_cta<T, R, MACROS, PART>(sd.a, sd.k);
+    rows_run<T, R, MACROS, PART>(sd.a, sd.k, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // A lone context steps rows in FP64 only: FP32 compute steps node pairs
@@ -383,6 +383,15 @@ __global__ void fields_to_compute_kernel(const double *const *out, R *rho, R *u,
 
 // ---- launchers ---------------------------------------------------------------
 
+// Block width of the per-node launch of a group's injector planes beside the row
+// kernel: whole warps along x, so that its plane sums land in the row kernel's
+// slots [y][x / 32] (the widest of 128, 96, 64 that divides NX, else 32 with a
+// partial last block).
+static int z0_block_x(int nx) {
+    for (int bx = 128; bx > 32; bx -= 32)
+        if (nx % bx == 0) return bx;
+    return 32;
+}
 // CTA width of the row kernel: NX rounded up to whole warps
 static int rows_block_x(int nx) { return (nx + 31) / 32 * 32; }
 
@@ -394,16 +403,20 @@ size_t lbm_rows_smem(int nx, size_t fsize, size_t gsize) {
 // per-node kernel measured faster (0.73 vs 0.76 ms at 256 x 256 x 129, FP16),
 // and FP32 compute with an even NX steps pairs (lbm_pair.cu), so that rows
 // serve FP64 and, in the grouped launches of a batch, FP32 and mixed storage
-// (2-byte f, 4-byte g).  Rows are whole bulk copies, so their bytes are
-// multiples of 16.
+// (2-byte f, 4-byte g), where they are the faster one on wide rows and many
+// instances: us a step grouped, rows / per-node, FP32 8 x 64 x 64 x 33 136 / 152,
+// 3 x 128 x 128 x 65 318 / 414, 2 x 64 x 64 x 33 57 / 49, 16 x 48 x 48 x 25 166 / 158;
+// mixed 6 x 96 x 96 x 49 308 / 317 (the autotuner tries both; a graph branch per
+// instance, with pairs, beats either: 97, 256, 38, 111, 235).  Rows are whole bulk
+// copies, so their bytes are multiples of 16.
 bool lbm_rows_usable(int nx, size_t fsize, size_t gsize) {
     return gsize >= 4 && nx >= 32 && nx <= 256 && (nx * fsize) % 16 == 0 &&
            (nx * gsize) % 16 == 0 && lbm_rows_smem(nx, fsize, gsize) <= 220 * 1024;
 }
 
 template <typename T, typename R>
-cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid) {
-    *grid = 0;
+cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid, int *group) {
+    *grid = *group = 0;
     using F = typename PopT<T>::F;
     using G = typename PopT<T>::G;
     if (!lbm_rows_usable(nx, sizeof(F), sizeof(G))) return cudaSuccess;
@@ -436,14 +449,15 @@ cudaError_t prepare_lbm_rows(int nx, int ny, int nz, int *grid) {
     auto run = [&](long long n) { return (rows + n - 1) / n; };
     const bool own = ny < slots && run(slots - ny) == run(slots);
     *grid = (int)std::min<long long>(rows, own ? slots - ny : slots);
+    *group = (int)std::min<long long>(rows, slots);
     return cudaSuccess;
 }
 
-template cudaError_t prepare_lbm_rows<double, double>(int, int, int, int *);
-template cudaError_t prepare_lbm_rows<float, float>(int, int, int, int *);
-template cudaError_t prepare_lbm_rows<__half, float>(int, int, int, int *);
-template cudaError_t prepare_lbm_rows<__nv_bfloat16, float>(int, int, int, int *);
-template cudaError_t prepare_lbm_rows<Mix16, float>(int, int, int, int *);
+template cudaError_t prepare_lbm_rows<double, double>(int, int, int, int *, int *);
+template cudaError_t prepare_lbm_rows<float, float>(int, int, int, int *, int *);
+template cudaError_t prepare_lbm_rows<__half, float>(int, int, int, int *, int *);
+template cudaError_t prepare_lbm_rows<__nv_bfloat16, float>(int, int, int, int *, int *);
+template cudaError_t prepare_lbm_rows<Mix16, float>(int, int, int, int *, int *);
 
 // ---- launches over a group of instances with the same grid ----------------
 //
@@ -496,14 +510,22 @@ cudaError_t launch_lbm_group(const void *desc_dev, int n, int nx, int ny, int nz
     return cudaGetLastError();
 }
 
-// The steady-state step of a group on the row kernel: per_inst CTAs walking
-// rows, and those of the injector plane, per instance.
+// The steady-state step of a group on the row kernel: plane z = 0 of every
+// instance on the per-node kernel (z0_block_x), then the planes z >= 1 on per_inst
+// CTAs of the row kernel per instance.  Two launches, unlike a lone context's one:
+// the injector CTAs of all instances, each holding a row walker's shared memory,
+// would take the slots of most walkers (us a step with one launch / two: 16 x 48 x
+// 48 x 25 in FP64 410 / 295, 6 x 96 x 96 x 49 in FP32 485 / 361, 8 x 64 x 64 x 33 mixed
+// 177 / 123).
 template <typename T, typename R>
 cudaError_t launch_lbm_rows_group(const void *desc_dev, int n, int nx, int ny, int per_inst,
                                   bool macros, cudaStream_t s) {
     const auto *d = reinterpret_cast<const LbmGroupDesc<T, R> *>(desc_dev);
     const size_t sm = lbm_rows_smem(nx, sizeof(typename PopT<T>::F), sizeof(typename PopT<T>::G));
-    const dim3 g1(ny + per_inst, n, 1);
+    const int bx = z0_block_x(nx);
+    const dim3 g0((nx + bx - 1) / bx, ny, n), g1(per_inst, n, 1);
+    if (macros) lbm_group_kernel<T, R, true><<<g0, bx, 0, s>>>(d, 1, 1);
+    else lbm_group_kernel<T, R, false><<<g0, bx, 0, s>>>(d, 1, 1);
     rows_group_kernel<T, R>(macros, nx % 32 != 0)<<<g1, rows_block_x(nx), sm, s>>>(d);
     return cudaGetLastError();
 }
