@@ -87,8 +87,13 @@ template <typename R>
 constexpr int min_blocks() { return sizeof(R) == 8 ? 2 : 3; }
 
 // The values of a in the order of the table's rows: all of them (odd n), or
-// the even ones, then the odd ones, each padded to whole stages.
-template <bool EVEN>
+// the even ones, then the odd ones, each padded to whole stages.  The inverse passes
+// (INV) take each of these runs from its end: their inputs are the modes of phi',
+// which fall off as a^-2, and a sum that adds the large ones last rounds at their
+// size once or twice instead of n / 4 times (E_x of a noisy charge in FP32, distance
+// from a 64-bit solve: 160 x 160 x 33 5.6e-6 the other way, 1.8e-6 so, radix passes
+// 2.7e-6; 360 x 90 x 20 9.2e-6, 2.1e-6 and 3.3e-6).
+template <bool EVEN, bool INV>
 struct Order {
     int n, te, ts;  // length, stages of the even values, all stages
     __device__ __forceinline__ explicit Order(int n_) : n(n_) {
@@ -96,10 +101,18 @@ struct Order {
         te = EVEN ? (h / 2 + 1 + kKC - 1) / kKC : (h + 1 + kKC - 1) / kKC;
         ts = EVEN ? te + ((h + 1) / 2 + kKC - 1) / kKC : te;
     }
-    // value of row r of stage t, and whether it exists
+    // table row of row r of stage t, its value, and whether it exists
+    __device__ __forceinline__ int row(int t, int r) const {
+        if (INV) {
+            t = t < te ? te - 1 - t : te + ts - 1 - t;
+            r = kKC - 1 - r;
+        }
+        return kKC * t + r;
+    }
     __device__ __forceinline__ int at(int t, int r) const {
-        if (!EVEN) return kKC * t + r;
-        return t < te ? 2 * (kKC * t + r) : 2 * (kKC * (t - te) + r) + 1;
+        const int i = row(t, r);
+        if (!EVEN) return i;
+        return i < kKC * te ? 2 * i : 2 * (i - kKC * te) + 1;
     }
     __device__ __forceinline__ bool in(int a) const { return 2 * a <= n; }
     __device__ __forceinline__ bool pair(int a) const { return a > 0 && 2 * a < n; }
@@ -156,11 +169,13 @@ template <int BN, typename R2>
 struct TableStage {
     static constexpr int kV = kKC * BN / kThreads;
     R2 v[kV];
-    __device__ __forceinline__ void load(const R2 *__restrict__ tab, int tp, int t, int n0) {
+    template <typename O>
+    __device__ __forceinline__ void load(const R2 *__restrict__ tab, int tp, const O &ord, int t,
+                                         int n0) {
 #pragma unroll
         for (int i = 0; i < kV; ++i) {
             const int e = threadIdx.x + kThreads * i, x = e / BN, k = e - x * BN;
-            v[i] = tab[(size_t)(kKC * t + x) * tp + n0 + k];
+            v[i] = tab[(size_t)ord.row(t, x) * tp + n0 + k];
         }
     }
     __device__ __forceinline__ void store(R2 *Bs) const {
@@ -220,7 +235,7 @@ dft_rows_fwd(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec,
     const int r0 = blockIdx.x * kM, n0 = blockIdx.y * BN;
     const bool sums = blockIdx.y == 0;
     const R ieps = (R)(1.0 / eps);
-    const Order<EVEN> ord(nx);
+    const Order<EVEN, false> ord(nx);
     q += (size_t)nx * ny;  // plane 1
     // staging: table row tid % 16 of the rows tid / 16 + 8 i
     const int xs = tid & 15, rs = tid >> 4;
@@ -245,7 +260,7 @@ dft_rows_fwd(const R *__restrict__ q, typename Cplx<R>::T *__restrict__ spec,
             lo[i] = in ? row[x] : qm[i];
             hi[i] = in && ord.pair(x) ? row[nx - x] : qm[i];
         }
-        tb.load(tab, tp, t, n0);
+        tb.load(tab, tp, ord, t, n0);
     };
     auto store = [&](int s, int t) {
         R2 *a = As + s * SA;
@@ -337,7 +352,7 @@ dft_rows_inv(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phip,
     R2 *Bs = As + 2 * SA;
     const int tid = threadIdx.x;
     const int r0 = blockIdx.x * kM, n0 = blockIdx.y * BN;
-    const Order<EVEN> ord(nx);
+    const Order<EVEN, true> ord(nx);
     const int ks = tid & 15, rs = tid >> 4;
     R2 v[4];
     TableStage<BN, R2> tb;
@@ -348,7 +363,7 @@ dft_rows_inv(const typename Cplx<R>::T *__restrict__ spec, R *__restrict__ phip,
             const int r = r0 + rs + 8 * i;
             v[i] = r < rows && ord.in(k) ? spec[(size_t)pitch * r + k] : zero2<R2>();
         }
-        tb.load(tab, tp, t, n0);
+        tb.load(tab, tp, ord, t, n0);
     };
     auto store = [&](int s, int t) {
         R2 *a = As + s * SA;
@@ -434,7 +449,7 @@ dft_cols(const typename Cplx<R>::T *__restrict__ in, typename Cplx<R>::T *__rest
     R2 *Bs = A2 + 2 * SA;                       // [2][kKC][BN]
     const int tid = threadIdx.x;
     const int m0 = (blockIdx.x % mtiles) * kM, n0 = (blockIdx.x / mtiles) * BN;
-    const Order<EVEN> ord(ny);
+    const Order<EVEN, (S > 0)> ord(ny);
     const size_t plane = (size_t)blockIdx.y * ny * pitch;
     in += plane;
     out += plane;
@@ -451,7 +466,7 @@ dft_cols(const typename Cplx<R>::T *__restrict__ in, typename Cplx<R>::T *__rest
             lo[i] = ok ? in[(size_t)pitch * y + m0 + cs] : zero2<R2>();
             hi[i] = ok && ord.pair(y) ? in[(size_t)pitch * (ny - y) + m0 + cs] : zero2<R2>();
         }
-        tb.load(tab, tp, t, n0);
+        tb.load(tab, tp, ord, t, n0);
     };
     auto store = [&](int s, int t) {
 #pragma unroll
