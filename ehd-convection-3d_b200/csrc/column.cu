@@ -72,10 +72,21 @@ __device__ __forceinline__ R dot_dir(int d, R a, R b, R c) {
     return s;
 }
 
-// Sum of the products sign(d) v_d, sign in {-1, 0, 1}, as a tree: a chain of
-// 27 FP64 additions would be the longest part of a step.
+// Sum of the products sign(d) v_d, sign in {-1, 0, 1}: in FP64 as a tree, a chain
+// of 27 FP64 additions being the longest part of a step otherwise; in FP32 in the
+// order of d, as the per-node kernel sums them (the tree's rounding took q, phi
+// and E 7, 12 and 12 % further from the 64-bit run over 800 columns of 13 to 49
+// planes, FP32 and mixed storage; in this order the distances are the per-node
+// kernel's, and mostly its bits).
 template <typename R, typename S>
-__device__ __forceinline__ R tree_sum(const R (&v)[Q], S sign) {
+__device__ __forceinline__ R dir_sum(const R (&v)[Q], S sign) {
+    if constexpr (sizeof(R) == 4) {
+        R a = 0;
+#pragma unroll
+        for (int d = 0; d < Q; ++d)
+            if (sign(d) != 0) a += sign(d) > 0 ? v[d] : -v[d];
+        return a;
+    }
     R t[Q];
     int n = 0;
 #pragma unroll
@@ -173,12 +184,12 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                 const R v = e == 0 ? s[d] : xf[mov_of(d) * nz + (e > 0 ? zm : zp)];
                 s[d] = v + c.w[cls_of(d)] * dr[e + 1];
             }
-            dev = tree_sum(s, [](int) { return 1; });
+            dev = dir_sum(s, [](int) { return 1; });
             rho = rref + dev;
             if (act) {
-                mom[z] = tree_sum(s, [](int d) { return ex_of(d); });
-                mom[nz + z] = tree_sum(s, [](int d) { return ey_of(d); });
-                mom[2 * nz + z] = tree_sum(s, [](int d) { return ez_of(d); });
+                mom[z] = dir_sum(s, [](int d) { return ex_of(d); });
+                mom[nz + z] = dir_sum(s, [](int d) { return ey_of(d); });
+                mom[2 * nz + z] = dir_sum(s, [](int d) { return ez_of(d); });
                 mom[3 * nz + z] = rho;
             }
         } else {
@@ -210,7 +221,7 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                     s[d] = v + c.w[cls_of(d)] * dq[e + 1];
                 }
             }
-            dev = tree_sum(s, [](int) { return 1; });
+            dev = dir_sum(s, [](int) { return 1; });
             charge = qref + dev;
             if (act) chg[z] = charge;
             // the warp's prefix sum of D and sum of (n + 1 - z) D
@@ -283,10 +294,19 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                     const R cu = dot_dir(d, tux, tuy, tuz);
                     const R eF = dot_dir(d, fx, (R)0, fz);
                     const R X = (R)0.5 * (s[d] + s[o]) + PK[q] - (R)0.5 * WR[q] * cu * cu;
-                    const R A = relax_rate(rp_hi, rp_lo, X) + QK[q] - c.c1[q] * cu * eF;
                     const R Y = (R)0.5 * (s[d] - s[o]) - WR[q] * cu;
-                    const R B = relax_rate(rm_hi, rm_lo, Y) - c.c2[q] * eF;
-                    const R od = s[d] - A - B, oo = s[o] - A + B;
+                    R od, oo;
+                    if (sizeof(R) == 4 && d != 5) {  // in the order of f_pair2
+                        const R A = fma(-c.c1[q], cu * eF, fma(rp_hi, X, fma(-rp_lo, X, QK[q])));
+                        const R B = fma(rm_hi, Y, fma(-rm_lo, Y, -c.c2[q] * eF));
+                        od = s[d] - (A + B);
+                        oo = (s[o] + B) - A;
+                    } else {
+                        const R A = relax_rate(rp_hi, rp_lo, X) + QK[q] - c.c1[q] * cu * eF;
+                        const R B = relax_rate(rm_hi, rm_lo, Y) - c.c2[q] * eF;
+                        od = s[d] - A - B;
+                        oo = s[o] - A + B;
+                    }
                     s[d] = od;
                     s[o] = oo;
                 }
@@ -341,6 +361,10 @@ column_steps_kernel(const ColumnArgs a, const KConst<R> c, int nsteps) {
                         const R t = (R)2 * WQ[q] * cu;
                         od = (s[o] + t) - A + cm_lo * Y;
                         oo = (s[d] - t) - A - cm_lo * Y;
+                    } else if (sizeof(R) == 4 && d != 5) {  // in the order of g_pair2
+                        const R B = relax_rate(cm_hi, cm_lo, Y);
+                        od = s[d] - (A + B);
+                        oo = (s[o] + B) - A;
                     } else {
                         const R B = relax_rate(cm_hi, cm_lo, Y);
                         od = s[d] - A - B;
