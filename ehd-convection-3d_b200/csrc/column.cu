@@ -11,7 +11,8 @@
 // included, 388 -> 26 ms (24.3 -> 1.6 us a step; 30 ms with the moments as
 // chains of additions and divisions by constants in the loop); 12 columns of
 // NZ = 25 as one batch, 12,000 steps, 609 -> 38 ms (one block per column, side
-// by side, where the batch's graph had held 84 launches a step).
+// by side, where the batch's graph had held 84 launches a step).  With one
+// multiprocessor busy the times scatter: other calls took up to 43 and 53 ms.
 //
 // Thread z of the first half of the block holds node z's flow populations f
 // in registers, thread z of the second half its charge populations g (the two

@@ -13,24 +13,25 @@
 // store.  Planes are walked as runs of node pairs, so that no lane is idle at
 // the end of a row.  That is 860 instructions a node; with the 168 registers
 // of three blocks a multiprocessor (12 warps) the step of 512 x 512 x 129 in
-// FP16 went 2.82 -> 2.15 ms (this kernel 1.65 ms; with two or four blocks,
+// FP16 went 2.82 -> 2.16 ms (this kernel 1.66 ms; with two or four blocks,
 // 255 or 128 registers, 2.62 and 2.66 ms), 256 x 256 x 129 in mixed storage
-// 0.690 -> 0.598 ms (there against the row kernel), 302 x 266 x 38 mixed 333 ->
-// 227 us for the LBM half.  What is left to the floor is load latency at that
+// 0.690 -> 0.586 ms (there against the row kernel), 302 x 266 x 38 mixed 333 ->
+// 210 us for the LBM half.  What is left to the floor is load latency at that
 // occupancy (2.3 of 5.7 cycles between issues).
 //
 // FP32 populations are 64-bit words: 760 instructions a node and 128 loads of
 // a thread in flight, where the row kernel of lbm.cu spends about 1,340 and its
 // warps wait on whole rows.  LBM half of a step in us, the kernel it replaced /
-// this: 256 x 256 x 129 663 / 579 (6.66 TB/s of its 456 B a node, the copy
-// bandwidth), 128 x 128 x 65 96.5 / 80.8, 64 x 64 x 33 13.5 / 11.0, 200 x 200 x
-// 65 241 / 196 (rows); 122 x 122 x 101 148 / 113, 302 x 266 x 38 301 / 232,
-// 512 x 512 x 33 764 / 615, 38 x 38 x 40 9.2 / 7.7 (one node per thread).
+// this: 256 x 256 x 129 663 / 582 (6.62 TB/s of its 456 algorithmic bytes a node,
+// 6.0 by the DRAM traffic), 128 x 128 x 65 96.5 / 83.2, 64 x 64 x 33 13.5 / 11.0,
+// 200 x 200 x 65 241 / 193 (rows); 122 x 122 x 101 148 / 118, 302 x 266 x 38 301 /
+// 232, 512 x 512 x 33 764 / 620, 38 x 38 x 40 9.2 / 7.5 (one node per thread).
 //
 // The injector plane z = 0 is stepped with one node per thread (node_step), by
 // blocks of the same launch in FP32 and on small grids, in a launch of its own
 // on large ones.  The pull, collision and wall rules are those of finish_node, on the
-// same deviations.  (Rows through shared memory, as in lbm_rows_kernel, with
+// same deviations and up to the plane sums in the same operations (rho and q of a
+// step are the same bits).  (Rows through shared memory, as in lbm_rows_kernel, with
 // g read twice to stay at 128 registers, took 2.53 ms where this takes 2.15.)
 #include <type_traits>
 

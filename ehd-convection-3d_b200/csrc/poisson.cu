@@ -19,10 +19,12 @@
 //   K3 z solve  : per (kx, ky) != (0,0), the tridiagonal system
 //                 phi(z-1) - (2 + k^2 dz^2) phi(z) + phi(z+1) = dz^2 s(z),
 //                 phi(0) = phi(NZ-1) = 0, in place: as a sine transform where
-//                 2(NZ-1) is a compile-time FFT size (poisson_zdst) and in BF16
-//                 contexts (poisson_zdst_rt), otherwise eliminated from both
-//                 ends in FP64 (poisson_zmeet), or by a one-sided sweep with a
-//                 pivot table where the tuning asks for it (poisson_zsolve).
+//                 2(NZ-1) is a compile-time FFT size (poisson_zdst), in BF16
+//                 contexts and on columns too tall for shared memory
+//                 (poisson_zdst_rt), otherwise eliminated from both ends in FP64
+//                 (poisson_zmeet), or by a one-sided sweep with a pivot table on
+//                 still taller ones and where the tuning asks for it
+//                 (poisson_zsolve).
 //                 The (0,0) mode in
 //                 FP64 from the plane sums plus NX NY q_m, with the electrode
 //                 voltage entering as -V/dz^2 on the plane z = 1
